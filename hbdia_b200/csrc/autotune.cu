@@ -114,9 +114,11 @@ void autotune(DevicePlan &P, const void *X, int64_t ldx, void *Y, int64_t ldy, i
                         cand.push_back(c);
                     }
             } else {
-                Choice c;
-                c.kernel = HBDIA_KERNEL_ROWWISE;
-                cand.push_back(c);
+                for (int32_t kern : {HBDIA_KERNEL_ROWWISE, HBDIA_KERNEL_QUAD}) {  // QUAD: the strip kernel, where it pays
+                    Choice c;
+                    c.kernel = kern;
+                    cand.push_back(c);
+                }
             }
         } else {
             for (int32_t t : {2, 4, 8, 16, 32}) {

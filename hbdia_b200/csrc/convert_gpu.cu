@@ -471,6 +471,7 @@ void convert_on_device(const Coo<T> &coo, int32_t bw, int32_t thr, int64_t maxCo
     const size_t oRP = carve((static_cast<size_t>(nR) + 1) * sizeof(int32_t));
     const size_t oTile = carve((static_cast<size_t>(Q.numTiles) + 1) * sizeof(int32_t));
     const size_t oStatus = carve(sizeof(int32_t));
+    const size_t oStrips = carve(strip_bytes(Q.numTiles));
     Q.bytes = off;
     check_cuda(dev_alloc(&Q.base, Q.bytes), "cudaMalloc(matrix layout)");
     try {
@@ -531,6 +532,7 @@ void convert_on_device(const Coo<T> &coo, int32_t bw, int32_t thr, int64_t maxCo
         int32_t nCooCheck = 0;
         check_cuda(cudaMemcpy(&nCooCheck, Q.cooRowPtr + nR, sizeof(int32_t), cudaMemcpyDeviceToHost), "cudaMemcpy");
         if (nCooCheck != nCoo) throw Error(HBDIA_ERR_RUNTIME, "device converter: COO count mismatch");
+        make_strips(Q, base + oStrips);
         cudaStream_t s;
         check_cuda(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), "cudaStreamCreate");
         Q.stream = s;

@@ -125,6 +125,10 @@ struct DevicePlan {
     int32_t *cooRow = nullptr, *cooCol = nullptr;
     void *cooVal = nullptr;              // T
     int32_t *cooRowPtr = nullptr, *cooTile = nullptr;
+    void *strips = nullptr;              // strip descriptors (spmv_strip.cuh); null: the strip kernel
+                                         // is not the faster one for this layout
+    int32_t stripGrid = 0;               // its CTAs
+    int32_t uniformStrips = 0;           // strips whose four tiles share one offset list
     void *stream = nullptr;              // cudaStream_t owned by the plan
     int32_t device = -1;                 // the device the layout lives on (current when it was built)
     void *xScratch = nullptr, *yScratch = nullptr;  // hbdia_spmv_host buffers
@@ -175,6 +179,13 @@ int32_t iteration_storage(const HostLayout<double> &L, int32_t storage);
 // A plan over a caller-owned device layout (layout_plan.cu).
 void borrow_plan(const hbdia_layout_desc &d, DevicePlan &P);
 void free_plan(DevicePlan &P);
+// Strip descriptors (strip.cu): their bytes in a plan's allocation, and making
+// them there from the layout on the device (P.strips: set where the strip
+// kernel pays).
+size_t strip_bytes(int32_t numTiles);
+void make_strips(DevicePlan &P, void *where);
+template <typename VT, typename XT>
+void launch_strip(const DevicePlan &P, const XT *x, XT *y, void *stream);
 // True when at least half of the stored offsets fall past the last full group
 // of the pipe kernel (histBlocks[d] = blocks with d offsets).
 bool tail_heavy(const std::vector<int32_t> &histBlocks);

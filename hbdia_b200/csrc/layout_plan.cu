@@ -6,8 +6,8 @@
 // row-sorted COO remainder with its CSR row pointer -- run through this
 // library's fused kernels without a copy.  The plan borrows those arrays and
 // owns only a small allocation: the COO range of every 32-row tile (derived
-// from the row pointer on the device) and the status word of the bounded
-// waits.
+// from the row pointer on the device), the strip descriptors (16 bytes per 128
+// rows) and the status word of the bounded waits.
 //
 // The arrays are checked on the device before the plan is returned (block
 // starts from 0 to totalOffsets and non-decreasing, the row pointer from 0 to
@@ -118,7 +118,8 @@ void borrow_plan(const hbdia_layout_desc &d, DevicePlan &P) {
     const size_t oTile = 0;
     const size_t oStatus = up256((static_cast<size_t>(Q.numTiles) + 1) * sizeof(int32_t));
     const size_t oFlags = oStatus + 256;
-    Q.bytes = oFlags + 256;
+    const size_t oStrips = oFlags + 256;
+    Q.bytes = oStrips + strip_bytes(Q.numTiles);
     check_cuda(dev_alloc(&Q.base, Q.bytes), "cudaMalloc(plan)");
     try {
         char *base = static_cast<char *>(Q.base);
@@ -142,6 +143,7 @@ void borrow_plan(const hbdia_layout_desc &d, DevicePlan &P) {
         tile_ranges<<<static_cast<unsigned>((Q.numTiles + 1 + 255) / 256), 256>>>(Q.cooRowPtr, Q.n, Q.numTiles,
                                                                                   Q.nCoo > 0, Q.cooTile);
         check_cuda(cudaGetLastError(), "tile_ranges");
+        make_strips(Q, base + oStrips);
         cudaStream_t s;
         check_cuda(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), "cudaStreamCreate");
         Q.stream = s;

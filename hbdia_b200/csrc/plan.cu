@@ -9,6 +9,7 @@
 //   cooRow/cooCol int32, cooVal T: the COO remainder, row-sorted (nCoo)
 //   cooRowPtr int32 CSR row pointer of the remainder            (numRows + 1)
 //   cooTile   int32 first remainder entry of each 32-row tile   (numTiles + 1)
+//   strips    16-byte descriptor of every 128 rows (spmv_strip.cuh)
 
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -239,6 +240,7 @@ void build_plan(const HostLayout<T> &L, int storage, DevicePlan &P, const Column
     const size_t oRP = carve((static_cast<size_t>(Q.n) + 1) * sizeof(int32_t));
     const size_t oTile = carve((static_cast<size_t>(Q.numTiles) + 1) * sizeof(int32_t));
     const size_t oStatus = carve(sizeof(int32_t));
+    const size_t oStrips = carve(strip_bytes(Q.numTiles));
     Q.bytes = off;
     check_cuda(dev_alloc(&Q.base, Q.bytes), "cudaMalloc(matrix layout)");
     char *base = static_cast<char *>(Q.base);
@@ -266,6 +268,7 @@ void build_plan(const HostLayout<T> &L, int storage, DevicePlan &P, const Column
         up(Q.cooVal, cv, Q.nCoo * sizeof(T));
         up(Q.cooRowPtr, crp, (static_cast<size_t>(Q.n) + 1) * sizeof(int32_t));
         up(Q.cooTile, tile.data(), (static_cast<size_t>(Q.numTiles) + 1) * sizeof(int32_t));
+        make_strips(Q, base + oStrips);
         cudaStream_t s;
         check_cuda(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), "cudaStreamCreate");
         Q.stream = s;
@@ -381,6 +384,9 @@ void launch_pipe(Kernel kernel, const dev::SpmvArgs<VT, XT> &a, int32_t numTiles
 // quad's values when x exceeds L2 (the pipelined kernel's rule).
 template <typename VT, typename XT>
 void launch_quad(const DevicePlan &P, const dev::SpmvArgs<VT, XT> &a, const XT *x, XT *y, cudaStream_t s) {
+    // narrow values without a knob set, wide blocks: the strip kernel where it pays
+    if (P.strips && (P.bw != 32 || (sizeof(VT) < sizeof(double) && P.dtype == HBDIA_F64 && !P.quadGroup && P.prefetchL2 < 0)))
+        return launch_strip<VT, XT>(P, x, y, s);
     int l2 = 0;
     const int device = plan_device(P);
     check_cuda(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, device), "cudaDeviceGetAttribute(L2)");
@@ -408,6 +414,9 @@ void launch_quad(const DevicePlan &P, const dev::SpmvArgs<VT, XT> &a, const XT *
 
 template <typename VT, typename XT>
 void launch_pipe_tuned(const DevicePlan &P, const dev::SpmvArgs<VT, XT> &a, const XT *x, XT *y, cudaStream_t s) {
+    // native values without a knob set: the strip kernel where it pays
+    if (P.strips && P.storage == HBDIA_STORE_NATIVE && P.prefetchL2 < 0 && P.maskedTail < 0 && P.unroll != 27)
+        return launch_strip<VT, XT>(P, x, y, s);
     // Forcing 4-6 CTAs per SM through __launch_bounds__ made ptxas spill and
     // ran 3-45% slower on B200; the compiler's own register choice is kept.
     // The prefetch pays when x does not fit in L2 (measured on B200: +1.5 % FP64
@@ -490,14 +499,16 @@ int32_t select_kernel(const DevicePlan &P, const void *x) {
             if (pipeOk) return HBDIA_KERNEL_PIPE;
             return bw32 ? HBDIA_KERNEL_WARP : HBDIA_KERNEL_ROWWISE;
         case HBDIA_KERNEL_QUAD:
-            if (pipeOk) return HBDIA_KERNEL_QUAD;
+            if (pipeOk || P.strips) return HBDIA_KERNEL_QUAD;
             return bw32 ? HBDIA_KERNEL_WARP : HBDIA_KERNEL_ROWWISE;
         case HBDIA_KERNEL_WARP: return bw32 ? HBDIA_KERNEL_WARP : HBDIA_KERNEL_ROWWISE;
         default:  // AUTO: the fastest measured on B200 for blockWidth 32
             // (4- and 2-byte values: the quad kernel, 2-10 % ahead of the
             // pipelined one on the 27-point 128^3 and 256^3 workloads; FP64
             // values: the pipelined kernel, which the quad one trails there)
+            // (both run as the strip kernel on layouts where that pays: strip.cu)
             if (pipeOk) return P.storage == HBDIA_STORE_NATIVE ? HBDIA_KERNEL_PIPE : HBDIA_KERNEL_QUAD;
+            if (P.strips) return HBDIA_KERNEL_QUAD;  // wide blocks
             return bw32 ? HBDIA_KERNEL_WARP : HBDIA_KERNEL_ROWWISE;
     }
 }

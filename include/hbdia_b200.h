@@ -70,7 +70,11 @@ typedef enum hbdia_value_storage {
 
 /* SpMV kernel choice (all give bit-identical y).  AUTO picks the kernel
  * measured fastest on B200: for blockWidth 32 QUAD with 4- and 2-byte value
- * storage, PIPE with 8-byte values; ROWWISE for other block widths.  STAGED
+ * storage, PIPE with native values; for other block widths QUAD when it is a
+ * multiple of 32 and the matrix is large and regular enough, else ROWWISE.
+ * PIPE (native values), QUAD (narrow ones, and wide blocks) run as the strip
+ * kernel, which streams the values of 4 blocks of 32 rows through shared
+ * memory, on layouts where that is the faster form.  STAGED
  * needs a 16-byte aligned x and value array (else WARP runs); PIPE and STAGED
  * need numRows <= 2^30. */
 typedef enum hbdia_kernel {
@@ -375,7 +379,8 @@ typedef struct hbdia_plan hbdia_plan;
  * valid and unchanged until hbdia_plan_destroy.  The arrays are checked on
  * the device first (block starts, row pointer, COO rows and columns);
  * HBDIA_ERR_INVALID_ARGUMENT / _OUT_OF_RANGE name what is malformed.  The
- * plan allocates only its per-tile COO ranges and a status word. */
+ * plan allocates only its per-tile COO ranges, 16 bytes per 128 rows and a
+ * status word. */
 int hbdia_plan_create(const hbdia_layout_desc *desc, hbdia_plan **out);
 /* hbdiaSpMV on the plan (the same fused kernels and bit-identical y as
  * hbdia_spmv_device on the matrix the layout came from); x holds
