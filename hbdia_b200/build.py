@@ -25,9 +25,9 @@ CUDA_HOME = os.environ.get("CUDA_HOME", "/usr/local/cuda")
 NVCC = os.path.join(CUDA_HOME, "bin", "nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
-CU_SOURCES = ["plan.cu", "autotune.cu", "cg.cu", "noalloc.cu", "batch.cu", "convert_gpu.cu", "halo.cu", "layout_plan.cu", "strip.cu"]
+CU_SOURCES = ["plan.cu", "autotune.cu", "cg.cu", "noalloc.cu", "batch.cu", "convert_gpu.cu", "halo.cu", "layout_plan.cu", "strip.cu", "spmm_rows.cu"]
 CPP_SOURCES = ["convert.cpp", "generate.cpp", "capi.cpp", "hbdia_cxx.cpp", "serve.cpp", "dia.cpp", "partition.cpp"]
-HEADERS = ["hbdia_internal.hpp", "spmv_kernels.cuh", "spmv_xstage.cuh", "spmv_quad.cuh", "spmv_strip.cuh", "spmm_kernels.cuh", "args.cuh",
+HEADERS = ["hbdia_internal.hpp", "spmv_kernels.cuh", "spmv_xstage.cuh", "spmv_quad.cuh", "spmv_strip.cuh", "spmm_kernels.cuh", "spmm_rows.cuh", "args.cuh",
            "batch_kernels.cuh", "handles.hpp"]
 
 

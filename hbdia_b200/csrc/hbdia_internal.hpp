@@ -198,6 +198,11 @@ void launch_spmm(const DevicePlan &P, const void *X, int64_t ldx, void *Y, int64
 void launch_spmm_tile(const DevicePlan &P, const void *X, int64_t ldx, void *Y, int64_t ldy, int32_t k,
                       int32_t tile, void *stream, bool colMajor = false);
 int32_t default_spmm_tile(int32_t k, bool colMajor = false);
+// Row-major Y = A X in passes of up to `width` columns, blockWidth a multiple
+// of 32 and numRows <= 2^30 (spmm_rows.cu).
+template <typename VT, typename XT>
+void launch_spmm_rows(const DevicePlan &P, const XT *X, int64_t ldx, XT *Y, int64_t ldy, int32_t k, int32_t width,
+                      void *stream);
 // k SpMVs of one matrix on separate device vectors (x[j] -> y[j]) as
 // vector-list SpMMs of up to 32 vectors per launch, bit-identical to k SpMVs.
 void launch_spmv_list(const DevicePlan &P, const void *const *x, void *const *y, int32_t k, void *stream);

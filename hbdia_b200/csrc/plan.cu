@@ -533,7 +533,10 @@ namespace {
 template <typename VT, typename XT, int KT, bool CM>
 void launch_spmm_kt(const DevicePlan &P, const dev::SpmvArgs<VT, XT> &a, const XT *X, int64_t ldx, XT *Y,
                     int64_t ldy, int32_t k, cudaStream_t s) {
-    if (P.bw == 32) {
+    if (P.bw == 32 && !CM) {  // only more than 2^30 rows come here: 64-bit indices
+        const unsigned grid = static_cast<unsigned>((static_cast<int64_t>(P.numTiles) + 7) / 8);
+        dev::spmm_bw32<VT, XT, KT, CM, int64_t, false><<<grid, 256, 0, s>>>(a, X, ldx, Y, ldy, k);
+    } else if (P.bw == 32) {
         const unsigned grid = static_cast<unsigned>((static_cast<int64_t>(P.numTiles) + 7) / 8);
         // The full passes in one launch, a partial last pass (k not a multiple
         // of KT) in a second one on the remaining columns; 32-bit gather
@@ -575,6 +578,7 @@ void launch_spmm_typed(const DevicePlan &P, const void *X, int64_t ldx, void *Y,
     const XT *xp = static_cast<const XT *>(X);
     XT *yp = static_cast<XT *>(Y);
     if (colMajor) launch_spmm_layout<VT, XT, true>(P, a, xp, ldx, yp, ldy, k, tile, s);
+    else if (P.bw % 32 == 0 && P.n <= (1 << 30)) launch_spmm_rows<VT, XT>(P, xp, ldx, yp, ldy, k, tile, s);
     else launch_spmm_layout<VT, XT, false>(P, a, xp, ldx, yp, ldy, k, tile, s);
     check_cuda(cudaGetLastError(), "SpMM launch");
 }
@@ -584,11 +588,11 @@ void launch_spmm_typed(const DevicePlan &P, const void *X, int64_t ldx, void *Y,
 int32_t default_spmm_tile(int32_t k, bool colMajor) {
     // Measured on B200 (27-point stencil 256^3): column-major blocks are
     // fastest in passes of 4 for every k >= 3 (each column a separate
-    // coalesced gather); row-major ones in the smallest tile covering k up to
-    // 8 (wider passes re-fetch the same lines of X in every pass).
+    // coalesced gather).  Row-major ones take whole rows of X, up to 32 columns
+    // a pass, so that every value is read once.
     if (k <= 2) return 2;
     if (colMajor || k <= 4) return 4;
-    return 8;
+    return k <= 8 ? 8 : k <= 16 ? 16 : 32;
 }
 
 void launch_spmm_tile(const DevicePlan &P, const void *X, int64_t ldx, void *Y, int64_t ldy, int32_t k,
