@@ -532,6 +532,7 @@ void convert_on_device(const Coo<T> &coo, int32_t bw, int32_t thr, int64_t maxCo
         int32_t nCooCheck = 0;
         check_cuda(cudaMemcpy(&nCooCheck, Q.cooRowPtr + nR, sizeof(int32_t), cudaMemcpyDeviceToHost), "cudaMemcpy");
         if (nCooCheck != nCoo) throw Error(HBDIA_ERR_RUNTIME, "device converter: COO count mismatch");
+        Q.tailHeavy = tail_heavy(meta.histBlocks);
         make_strips(Q, base + oStrips);
         cudaStream_t s;
         check_cuda(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), "cudaStreamCreate");
@@ -547,7 +548,6 @@ void convert_on_device(const Coo<T> &coo, int32_t bw, int32_t thr, int64_t maxCo
     if (Q.scale) bytes += 4 * static_cast<int64_t>(nb);
     if (Q.nCoo > 0) bytes += bw == 32 ? 4 * (static_cast<int64_t>(Q.numTiles) + 1) : 4 * (static_cast<int64_t>(nR) + 1);
     Q.bytesPerSpmv = bytes;
-    Q.tailHeavy = tail_heavy(meta.histBlocks);
     P = Q;
 }
 

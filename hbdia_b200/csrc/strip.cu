@@ -45,28 +45,40 @@ void configure(const DevicePlan &P) {
     });
 }
 
-// Whether the strip kernel is the faster one for a layout (B200, us):
-//  * it needs enough strips for the SMs' 2368 warps, since a warp's first strip
-//    waits for a chain of loads that the other kernels spread over four times
-//    as many warps.  Native values of blockWidth 32 against the pipelined
-//    kernel: 27-point FP64 80^3 (1.7 strips per warp) 27.9 against 24.8, 96^3
-//    (2.9) 38.9 against 38.4, 112^3 (4.6) 60.0 against 61.7; float 80^3 20.6
-//    against 18.6.  FP32 storage against the quad kernel: 40^3 (0.2) 14.4
-//    against 12.4, 56^3 (0.6) 14.4 against 17.9; BF16 storage 64^3 (0.9) 18.5
-//    against 17.1, 80^3 25.0 against 26.6.  Wide blocks against the
-//    row-per-thread kernel: 32^3 (0.1) 14.4 against 12.4, 64^3 (0.9) 20.7
-//    against 22.6;
-//  * most strips must share one list: 27-point 300x4x1000 (75 % do) 53.7
-//    against 45.6, 20x20x2000 (99 %) 34.1 against 36.0, 40^3 (88 %);
-//  * 16-byte copies need a 16-byte aligned value array (a caller's may not be).
-bool strip_pays(const DevicePlan &P, int sms) {
+// Whether a layout has enough work for the strip kernel to be the faster one.
+// A warp's first strip waits for a chain of loads that the other kernels spread
+// over four times as many warps (148 x 16 here).  B200, us, other kernel ->
+// strip kernel:
+//  * native values of blockWidth 32, from 4 strips a warp: 27-point FP64 80^3
+//    (1.7) 24.8 -> 27.9, 96^3 (2.9) 38.4 -> 38.9, 112^3 (4.6) 61.7 -> 60.0; 9
+//    offsets 950 K rows (3.1) 20.9 -> 21.6, 1.5 M (4.9) 31.6 -> 26.7, float
+//    16.5 -> 17.3, 24.4 -> 20.5.  From 2 where the pipelined kernel's groups of
+//    9 are mostly tails: 7-point 64^3 (0.9) 8.7 -> 10.3, 90^3 (2.4) 22.6 ->
+//    17.8, 100^3 (3.3) 28.7 -> 20.6, float 22.9 -> 16.9;
+//  * FP32 storage, from half a strip a warp and 32 K strip-offsets: 27-point
+//    40^3 (13 K) 12.4 -> 14.4, 56^3 (37 K) 17.9 -> 14.4; 9 offsets 280 K rows
+//    (20 K) 8.4 -> 9.5, 600 K (42 K) 13.3 -> 13.7, 1 M 19.9 -> 18.5; 7-point
+//    70^3 (19 K) 11.0 -> 12.3, 80^3 (28 K) 16.0 -> 12.4;
+//  * BF16 storage, from 1.5 and 48 K: 27-point 64^3 (0.9) 17.1 -> 18.5, 80^3
+//    (1.7, 108 K) 26.6 -> 25.0; 9 offsets 500 K rows (35 K) 12.3 -> 14.3, 800 K
+//    (56 K) 16.2 -> 16.5, 1.5 M 26.6 -> 22.9; 7-point 80^3 (28 K) 12.8 -> 14.4,
+//    96^3 (48 K) 17.3 -> 16.5;
+//  * wide blocks, from half a strip a warp: 27-point blockWidth 64 32^3 (0.1)
+//    12.4 -> 14.4, 45^3 (0.3) equal, 64^3 (0.9) 22.6 -> 20.7.
+// 16-byte copies need a 16-byte aligned value array (a caller's may not be).
+bool enough_strips(const DevicePlan &P, int sms) {
     const int64_t strips = (static_cast<int64_t>(P.numTiles) + 3) / 4, warps = int64_t(sms) * kStripWarps;
     const bool native = P.storage == HBDIA_STORE_NATIVE, bf16 = P.storage == HBDIA_STORE_BF16_SCALED;
     if (P.bw % 32 != 0 || P.n > (1 << 30) || (bf16 && P.bw != 32)) return false;
     if ((reinterpret_cast<uintptr_t>(P.vals) & 15) != 0) return false;
-    const int64_t least = native && P.bw == 32 ? 3 * warps : bf16 ? warps * 3 / 2 : warps / 2;
-    return strips >= least && P.uniformStrips >= 0.85 * static_cast<double>(strips);
+    if (native) return strips >= (P.bw != 32 ? warps / 2 : P.tailHeavy ? 2 * warps : 4 * warps);
+    const int64_t stripOffsets = P.totalOffsets * (P.bw / 32) / 4;
+    return bf16 ? strips >= warps * 3 / 2 && stripOffsets >= 48 * 1024 : strips >= warps / 2 && stripOffsets >= 32 * 1024;
 }
+
+// The least share of strips with one list: 27-point 300x4x1000 (75 %) 45.6 ->
+// 53.7 us, 20x20x2000 (99 %) 36.0 -> 34.1.
+constexpr double kUniformShare = 0.85;
 
 }  // namespace
 
@@ -76,7 +88,10 @@ void make_strips(DevicePlan &P, void *where) {
     P.strips = nullptr;
     P.stripGrid = 0;
     P.uniformStrips = 0;
-    if (P.bw % 32 != 0 || P.numTiles <= 0) return;
+    int device = 0, sms = 0;
+    check_cuda(cudaGetDevice(&device), "cudaGetDevice");
+    check_cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device), "cudaDeviceGetAttribute");
+    if (!enough_strips(P, sms)) return;
     const int32_t strips = (P.numTiles + 3) / 4;
     int4 *desc = static_cast<int4 *>(where);
     int32_t *uniform = reinterpret_cast<int32_t *>(desc + strips);
@@ -85,10 +100,7 @@ void make_strips(DevicePlan &P, void *where) {
         P.blkOff, P.offs, P.cooTile, P.numBlocks, P.numTiles, P.bw / 32, P.nCoo > 0, desc, uniform);
     check_cuda(cudaGetLastError(), "strip descriptors");
     check_cuda(cudaMemcpy(&P.uniformStrips, uniform, sizeof(int32_t), cudaMemcpyDeviceToHost), "cudaMemcpy(strips)");
-    int device = 0, sms = 0;
-    check_cuda(cudaGetDevice(&device), "cudaGetDevice");
-    check_cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device), "cudaDeviceGetAttribute");
-    if (!strip_pays(P, sms)) return;
+    if (P.uniformStrips < kUniformShare * strips) return;
     P.strips = desc;
     P.stripGrid = static_cast<int32_t>(std::min<int64_t>((strips + kStripWarps - 1) / kStripWarps, sms));
     // here and not at the launch, which may be captured into a graph

@@ -43,16 +43,21 @@ def _matrix(n, K, seed):
     return rows[o].astype(np.int32), cols[o].astype(np.int32), vals[o], x
 
 
-NATIVE, HALF, WIDE = 7104 * 128, 1184 * 128, 3552 * 128  # the fewest rows of each on 148 SMs
+# Rows from which the layouts below run the strip kernel on 148 SMs: native values (fewer where lists are short);
+# wide blocks; and FP32 / BF16 storage, whose lists count too
+NATIVE, SHORT, HALF = 9472 * 128, 4736 * 128, 1184 * 128
+def _fp32(K): return max(HALF, -(-32 * 1024 // K) * 128 * 21 // 20)
+def _bf16(K): return max(3552 * 128, -(-48 * 1024 // K) * 128 * 21 // 20)
 
 
 @pytest.mark.parametrize("storage,dtype,bw,n,K", [
-    ("STORE_NATIVE", "f8", 32, NATIVE + 77, 3), ("STORE_NATIVE", "f8", 32, NATIVE, 9),
-    ("STORE_NATIVE", "f4", 32, NATIVE + 1, 6), ("STORE_NATIVE", "f8", 64, HALF + 45, 7),
+    ("STORE_NATIVE", "f8", 32, SHORT + 77, 3), ("STORE_NATIVE", "f8", 32, NATIVE, 9),
+    ("STORE_NATIVE", "f4", 32, SHORT + 1, 6), ("STORE_NATIVE", "f8", 64, HALF + 45, 7),
     ("STORE_NATIVE", "f8", 96, HALF + 200, 4), ("STORE_NATIVE", "f4", 64, HALF + 33, 5),
-    ("STORE_F32", "f8", 32, HALF + 45, 1), ("STORE_F32", "f8", 32, HALF + 96, 31), ("STORE_F32", "f8", 64, HALF + 64, 8),
-    ("STORE_F32_QUAD", "f8", 32, HALF + 45, 10), ("STORE_F32_QUAD", "f8", 32, HALF + 31, 32),
-    ("STORE_BF16_SCALED", "f8", 32, WIDE + 45, 7), ("STORE_BF16_QUAD", "f8", 32, WIDE + 127, 5)])
+    ("STORE_F32", "f8", 32, _fp32(4) + 45, 4), ("STORE_F32", "f8", 32, _fp32(31) + 96, 31),
+    ("STORE_F32", "f8", 64, _fp32(8) + 64, 8), ("STORE_F32_QUAD", "f8", 32, _fp32(10) + 45, 10),
+    ("STORE_F32_QUAD", "f8", 32, _fp32(32) + 31, 32), ("STORE_BF16_SCALED", "f8", 32, _bf16(7) + 45, 7),
+    ("STORE_BF16_QUAD", "f8", 32, _bf16(13) + 127, 13)])
 def test_strip_equals_oracle(lib, storage, dtype, bw, n, K):
     import oracle
     rows, cols, vals, x = _matrix(n, K, K + bw)
