@@ -75,7 +75,7 @@ def measured_peak():
 def profiled_traffic():
     """Per-launch DRAM bytes of the SpMV kernel from the committed ncu summary
     (line 'traffic_bytes_per_launch: N')."""
-    p = os.path.join(ROOT, "profiles", "spmv_bw32_pipe_fp64_stencil27_256cube.md")
+    p = os.path.join(ROOT, "profiles", "spmv_strip_stencil27_128cube.md")
     try:
         with open(p) as f:
             for line in f:
