@@ -73,21 +73,16 @@ __device__ __forceinline__ void cp_async_wait_upto(int pending) {
     }
 }
 
-// N list entries, four (or two) at a time; the list is 16-byte aligned there.
-template <int N, bool V4>
+// N list entries, four at a time; the list is 16-byte aligned there.
+template <int N>
 __device__ __forceinline__ void load_list(const int32_t *p, int32_t (&o)[N]) {
-    if constexpr (V4) {
 #pragma unroll
-        for (int u = 0; u < N; u += 4) {
-            const int4 t = *reinterpret_cast<const int4 *>(p + u);
-            o[u] = t.x; o[u + 1] = t.y; o[u + 2] = t.z; o[u + 3] = t.w;
-        }
-    } else {
-#pragma unroll
-        for (int u = 0; u < N; u += 2) {
-            const int2 t = *reinterpret_cast<const int2 *>(p + u);
-            o[u] = t.x; o[u + 1] = t.y;
-        }
+    for (int u = 0; u < N; u += 4) {
+        const int4 t = *reinterpret_cast<const int4 *>(p + u);
+        o[u] = t.x;
+        o[u + 1] = t.y;
+        o[u + 2] = t.z;
+        o[u + 3] = t.w;
     }
 }
 
@@ -160,7 +155,7 @@ spmv_strip(const SpmvArgs<VT, XT> a, const int4 *__restrict__ desc, const XT *__
     constexpr int PB = QL ? 512 : 128;                     // contiguous bytes per tile and copy instruction
     constexpr int NI = (GB + 511) / 512;
     constexpr int WU = 4 * U;  // offsets of one tile per stage when the tiles differ
-    static_assert(U == 2 || U == 4, "groups of two or four offsets");
+    static_assert(U == 4, "the list is read four offsets at a time");
     static_assert(B32 || PB <= RB, "a copy instruction stays within one row");
     extern __shared__ __align__(16) unsigned char smem[];
     const int lane = threadIdx.x & 31;
@@ -382,9 +377,8 @@ spmv_strip(const SpmvArgs<VT, XT> a, const int4 *__restrict__ desc, const XT *__
                 constexpr bool CK = decltype(CHECK)::value;
                 XT xv[C][4];
                 unsigned ok = 0;
-                constexpr int CV = U % 4 == 0 ? (C + 3) / 4 * 4 : U;
-                int32_t of[CV];
-                load_list<CV, U % 4 == 0>(so + g, of);
+                int32_t of[(C + 3) / 4 * 4];
+                load_list(so + g, of);
 #pragma unroll
                 for (int u = 0; u < C; ++u) {
                     const XT *xp = xr + of[u];
@@ -427,10 +421,8 @@ spmv_strip(const SpmvArgs<VT, XT> a, const int4 *__restrict__ desc, const XT *__
 #pragma unroll 1
                 for (; g + U <= K; g += U) step(std::integral_constant<int, U>(), CHECK, g);
                 const int32_t rest = K - g;
-                if constexpr (U > 3)
-                    if (rest == 3) step(std::integral_constant<int, 3>(), CHECK, g);
-                if constexpr (U > 2)
-                    if (rest == 2) step(std::integral_constant<int, 2>(), CHECK, g);
+                if (rest == 3) step(std::integral_constant<int, 3>(), CHECK, g);
+                if (rest == 2) step(std::integral_constant<int, 2>(), CHECK, g);
                 if (rest == 1) step(std::integral_constant<int, 1>(), CHECK, g);
             };
             if (interior) all(std::false_type());
