@@ -326,8 +326,14 @@ spmm_rows(const SpmvArgs<VT, XT> a, const XT *__restrict__ X, int64_t ldx, XT *_
 #pragma unroll
                 for (int v = 0; v < V; ++v) acc[t][v] = XT(0);
             rows_dia<VT, XT, V, G, S>(a, xb, ldx, mt, first, vp, sc, row0, row, lane, vec, acc);
-            if (mt.c1 > mt.c0)
+            if (mt.c1 > mt.c0) {
                 rows_coo<VT, XT, V, G, S>(a, X + c0 + cx, ldx, mt.c0, mt.c1, row0, cr, cc, cv, lane, coo[threadIdx.x >> 5], acc);
+            } else if (a.hasCoo) {  // rows without entries add an empty sum: -0 becomes +0
+#pragma unroll
+                for (int t = 0; t < S; ++t)
+#pragma unroll
+                    for (int v = 0; v < V; ++v) acc[t][v] = add_rn(acc[t][v], XT(0));
+            }
             if (on) {
 #pragma unroll
                 for (int t = 0; t < S; ++t)

@@ -44,9 +44,9 @@
 // Arithmetic is the reference's, in the reference's order: per row, offsets
 // ascending, stored zeros and columns outside [0, xn) skipped, fma; COO
 // products summed from zero in list order with separately rounded multiply
-// and add; y = dia + coo for rows with remainder entries, y = dia otherwise
-// (src/Operations/HBDIASpMV.cu:42-88, src/Operations/HBDIASpMV.cpp:76-92).
-// (dia + 0 would equal dia: the FMA chain from +0 never yields -0.)
+// and add; y = dia + coo when the matrix has a remainder (+0 is added at rows
+// without entries: a chain of products that underflow can end in -0), else
+// y = dia (src/Operations/HBDIASpMV.cu:42-88, src/Operations/HBDIASpMV.cpp:76-92).
 #pragma once
 
 #include "spmv_kernels.cuh"
@@ -336,9 +336,11 @@ spmv_bw32_quad(const SpmvArgs<VT, XT> a, const XT *__restrict__ x, XT *__restric
             for (int q = 0; q < 4; ++q)
                 if (kq[q + 1] > kq[q]) sum[q] = block_dia<VT, XT>(a, x, kq[q], kq[q + 1], row + 32 * q, lane, sc[q]);
         }
-        // COO remainder: the heads of row segments add their sums into db
+        // COO remainder: every row's sum starts from +0 (a row's own sum is never
+        // -0, so adding the +0 first leaves rows with entries as they are);
+        // the heads of row segments add their sums into db
 #pragma unroll
-        for (int q = 0; q < 4; ++q) db[lane + 32 * q] = sum[q];
+        for (int q = 0; q < 4; ++q) db[lane + 32 * q] = a.hasCoo ? add_rn(sum[q], XT(0)) : sum[q];
         __syncwarp();
         const int32_t c0 = cq[0], c4 = cq[4];
         if (c4 > c0) {

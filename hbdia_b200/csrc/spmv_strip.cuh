@@ -38,7 +38,8 @@
 // Arithmetic is the reference's, in the reference's order: per row, offsets
 // ascending, stored zeros and columns outside [0, xn) skipped, fma; COO
 // products summed from zero in list order with separately rounded multiply
-// and add; y = dia + coo for rows with remainder entries, y = dia otherwise
+// and add; y = dia + coo when the matrix has a remainder (+0 is added at rows
+// without entries, which turns a sum of -0 into +0), else y = dia
 // (src/Operations/HBDIASpMV.cu:42-88, src/Operations/HBDIASpMV.cpp:76-92).
 #pragma once
 
@@ -463,7 +464,13 @@ spmv_strip(const SpmvArgs<VT, XT> a, const int4 *__restrict__ desc, const XT *__
             }
         }
 
-        // COO remainder: the heads of row segments add their sums into db
+        // COO remainder: every row's sum starts from +0 (a row's own sum is never
+        // -0, so adding the +0 first leaves rows with entries as they are);
+        // the heads of row segments add their sums into db
+        if (a.hasCoo) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) sum[q] = add_rn(sum[q], XT(0));
+        }
         if (c1 > c0) {
 #pragma unroll
             for (int q = 0; q < 4; ++q) db[lane + 32 * q] = sum[q];
