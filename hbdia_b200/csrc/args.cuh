@@ -25,6 +25,7 @@ inline dev::SpmvArgs<VT, XT> make_args(const DevicePlan &P) {
     a.numTiles = P.numTiles;
     a.hasCoo = P.nCoo > 0;
     a.quadLayout = P.quadLayout ? 1 : 0;
+    a.ascending = P.ascending ? 1 : 0;
     return a;
 }
 

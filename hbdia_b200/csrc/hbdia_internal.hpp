@@ -125,6 +125,7 @@ struct DevicePlan {
     int32_t *cooRow = nullptr, *cooCol = nullptr;
     void *cooVal = nullptr;              // T
     int32_t *cooRowPtr = nullptr, *cooTile = nullptr;
+    bool ascending = true;               // every block's offsets ascend (a caller's may not: layout_plan.cu)
     void *strips = nullptr;              // strip descriptors (spmv_strip.cuh); null: the strip kernel
                                          // is not the faster one for this layout
     int32_t stripGrid = 0;               // its CTAs

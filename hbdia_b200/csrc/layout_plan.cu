@@ -13,8 +13,10 @@
 // starts from 0 to totalOffsets and non-decreasing, the row pointer from 0 to
 // numCoo and non-decreasing, every COO row consistent with it and every COO
 // column inside the matrix), so a malformed layout is refused instead of
-// being read out of bounds.  Offsets need no check: the kernels bound every
-// column.
+// being read out of bounds.  Offsets may have any values: the kernels bound
+// every column, and where they do so by a list's first and last offset
+// (interior tiles) they need to know that the lists ascend, which is found here
+// (DevicePlan::ascending).  Lists that do not are summed in list order.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -58,6 +60,17 @@ __global__ void check_layout(const int32_t *__restrict__ blk, int32_t nb, int64_
         }
     }
     if (f) atomicOr(flags, f);
+}
+
+// *flags |= 1 when some block's offsets do not ascend.
+__global__ void check_order(const int32_t *__restrict__ blk, const int32_t *__restrict__ offs, int32_t nb,
+                            int32_t *__restrict__ flags) {
+    const int64_t b = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (b >= nb) return;
+    int32_t f = 0;
+    const int32_t k1 = blk[b + 1];
+    for (int32_t k = blk[b] + 1; k < k1; ++k) f |= offs[k - 1] > offs[k];
+    if (f) atomicOr(flags, 1);
 }
 
 // cooTile[t] = rowPtr[min(32 t, n)]: the COO range of each 32-row tile.
@@ -143,6 +156,12 @@ void borrow_plan(const hbdia_layout_desc &d, DevicePlan &P) {
         tile_ranges<<<static_cast<unsigned>((Q.numTiles + 1 + 255) / 256), 256>>>(Q.cooRowPtr, Q.n, Q.numTiles,
                                                                                   Q.nCoo > 0, Q.cooTile);
         check_cuda(cudaGetLastError(), "tile_ranges");
+        if (Q.numBlocks > 0) {  // (the flags are all zero here, and the block starts valid)
+            check_order<<<static_cast<unsigned>((Q.numBlocks + 255) / 256), 256>>>(Q.blkOff, Q.offs, Q.numBlocks, flags);
+            check_cuda(cudaGetLastError(), "check_order");
+            check_cuda(cudaMemcpy(&f, flags, sizeof(int32_t), cudaMemcpyDeviceToHost), "cudaMemcpy(flags)");
+            Q.ascending = f == 0;
+        }
         make_strips(Q, base + oStrips);
         cudaStream_t s;
         check_cuda(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), "cudaStreamCreate");

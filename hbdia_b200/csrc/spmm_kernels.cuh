@@ -140,7 +140,7 @@ __device__ __forceinline__ void spmm_pass(const SpmvArgs<VT, XT> &a, const XS &x
         const int32_t myoff = lane < cnt ? __ldg(a.offs + kb + lane) : 0;
         const VT *vp = a.vals + static_cast<int64_t>(kb) * 32 + lane;
         const int32_t offFirst = __shfl_sync(kFull, myoff, 0), offLast = __shfl_sync(kFull, myoff, cnt - 1);
-        if (row0 + offFirst >= 0 && row0 + 31 + offLast < a.xn)
+        if (a.ascending && row0 + offFirst >= 0 && row0 + 31 + offLast < a.xn)
             spmm_chunk<VT, XT, KT, IT, FULL, false>(a, xs, vp, myoff, cnt, row, kc, s, acc);
         else
             spmm_chunk<VT, XT, KT, IT, FULL, true>(a, xs, vp, myoff, cnt, row, kc, s, acc);

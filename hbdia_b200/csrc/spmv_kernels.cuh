@@ -47,6 +47,7 @@ struct SpmvArgs {
     int32_t numTiles;        // ceil(n / 32)
     int32_t hasCoo;          // COO remainder non-empty
     int32_t quadLayout;      // 4- / 2-byte values of uniform quads interleaved (spmv_quad.cuh)
+    int32_t ascending;       // every block's offsets ascend: a list's first and last bound the others
 };
 
 __device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
@@ -279,7 +280,7 @@ spmv_bw32_pipe(const SpmvArgs<VT, XT> a, const XT *__restrict__ x, XT *__restric
         // co-limits the kernel; the 8-byte instance is bandwidth-bound and the
         // extra path would cost it registers (80 instead of 64: fewer warps).
         const int32_t K = m.k1 - m.k0;
-        const bool interior = sizeof(VT) < 8 && K > 0 && K <= 32 && row0 + __shfl_sync(kFull, myoff, 0) >= 0 &&
+        const bool interior = sizeof(VT) < 8 && a.ascending && K > 0 && K <= 32 && row0 + __shfl_sync(kFull, myoff, 0) >= 0 &&
                               static_cast<int64_t>(row0) + 31 + __shfl_sync(kFull, myoff, K > 0 && K <= 32 ? K - 1 : 0) <
                                   static_cast<int64_t>(a.xn);
         const XT *xr = x + row;

@@ -312,7 +312,7 @@ spmv_bw32_quad(const SpmvArgs<VT, XT> a, const XT *__restrict__ x, XT *__restric
             if (K > 0) {
                 const int32_t offFirst = __shfl_sync(kFull, cur.myoff, 0);
                 const int32_t offLast = __shfl_sync(kFull, cur.myoff, K - 1);
-                const bool interior = int64_t(row0) + offFirst >= 0 && int64_t(row0) + 127 + offLast < int64_t(a.xn);
+                const bool interior = a.ascending && int64_t(row0) + offFirst >= 0 && int64_t(row0) + 127 + offLast < int64_t(a.xn);
                 bool done = false;
                 if constexpr (sizeof(VT) < 8) {
                     if (a.quadLayout) {  // interleaved region of the quad

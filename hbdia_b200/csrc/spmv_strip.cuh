@@ -371,7 +371,7 @@ spmv_strip(const SpmvArgs<VT, XT> a, const int4 *__restrict__ desc, const XT *__
             }
         }
         if (K > 0) {
-            const bool interior = int64_t(row0) + so[0] >= 0 && int64_t(row0) + 127 + so[K - 1] < int64_t(a.xn);
+            const bool interior = a.ascending && int64_t(row0) + so[0] >= 0 && int64_t(row0) + 127 + so[K - 1] < int64_t(a.xn);
             // C offsets from g on: their x first, then their values
             auto step = [&](auto CNT, auto CHECK, int32_t g) {
                 constexpr int C = decltype(CNT)::value;

@@ -307,7 +307,7 @@ spmv_bw32_xs(const XsArgs<VT, XT> A, const XT *__restrict__ x, XT *__restrict__ 
         const int32_t row = row0 + lane;
         // interior tile (every column of every offset inside [0, xn), at most
         // 32 offsets): no column checks, x read at x + row + offset
-        const bool interior = K > 0 && K <= 32 && int64_t(row0) + H.off[0] >= 0 &&
+        const bool interior = a.ascending && K > 0 && K <= 32 && int64_t(row0) + H.off[0] >= 0 &&
                               int64_t(row0) + 31 + H.off[K - 1] < int64_t(a.xn);
         // this tile's x gathers, all in flight before the wait
         XT xv[32];
