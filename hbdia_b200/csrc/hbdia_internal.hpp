@@ -129,7 +129,6 @@ struct DevicePlan {
     void *strips = nullptr;              // strip descriptors (spmv_strip.cuh); null: the strip kernel
                                          // is not the faster one for this layout
     int32_t stripGrid = 0;               // its CTAs
-    int32_t uniformStrips = 0;           // strips whose four tiles share one offset list
     void *stream = nullptr;              // cudaStream_t owned by the plan
     int32_t device = -1;                 // the device the layout lives on (current when it was built)
     void *xScratch = nullptr, *yScratch = nullptr;  // hbdia_spmv_host buffers

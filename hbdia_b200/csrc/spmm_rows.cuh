@@ -207,7 +207,7 @@ __device__ __forceinline__ void rows_dia(const SpmvArgs<VT, XT> &a, const XT *__
 #pragma unroll
                 for (int l = 0; l < GL; ++l)
                     ld_values<VT, S>(vp + static_cast<int64_t>(kb - mt.k0 + j + l0 + l) * a.bw, vec, vs[l]);
-                bool nz = VOTE;
+                bool nz = VOTE && (sizeof(VT) != 2 || sc != 0.0f);  // (scale 0: every widened value is zero)
                 if constexpr (VOTE) {
 #pragma unroll
                     for (int l = 0; l < GL; ++l)

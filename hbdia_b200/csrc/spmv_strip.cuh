@@ -90,11 +90,13 @@ __device__ __forceinline__ void load_list(const int32_t *p, int32_t (&o)[N]) {
 // One strip (4 consecutive 32-row tiles), made once per layout: x = first
 // offset index of the first tile's block; y = number of offsets when the four
 // tiles share one list of at most 32 offsets, else -1; z, w = the strip's COO
-// entries [z, w).
+// entries [z, w).  counts[0]: strips of one list; counts[1]: not zero when a
+// block's scale is 0, infinite or NaN (add_product tells zeros by the stored
+// value, which then is not what the widened one says).
 inline __global__ void __launch_bounds__(256)
 strip_desc_kernel(const int32_t *__restrict__ blkOff, const int32_t *__restrict__ offs,
-                  const int32_t *__restrict__ cooTile, int32_t numBlocks, int32_t numTiles, int32_t tilesPerBlock,
-                  int32_t hasCoo, int4 *__restrict__ desc, int32_t *__restrict__ uniform) {
+                  const int32_t *__restrict__ cooTile, const float *__restrict__ scale, int32_t numBlocks, int32_t numTiles,
+                  int32_t tilesPerBlock, int32_t hasCoo, int4 *__restrict__ desc, int32_t *__restrict__ counts) {
     const int lane = threadIdx.x & 31;
     const int32_t s = static_cast<int32_t>((static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x) >> 5);
     const int32_t numStrips = (numTiles + 3) / 4;
@@ -117,7 +119,14 @@ strip_desc_kernel(const int32_t *__restrict__ blkOff, const int32_t *__restrict_
         d.z = hasCoo ? cooTile[min(s * 4, numTiles)] : 0;
         d.w = hasCoo ? cooTile[min(s * 4 + 4, numTiles)] : 0;
         desc[s] = d;
-        if (uni) atomicAdd(uniform, 1);
+        if (uni) atomicAdd(counts, 1);
+        if (scale)
+            for (int i = 0; i < 4; ++i) {
+                const int32_t b = (s * 4 + i) / tilesPerBlock;
+                if (b >= numBlocks) break;
+                const float sc = fabsf(scale[b]);
+                if (!(sc > 0.0f && sc < __int_as_float(0x7f800000))) atomicOr(counts + 1, 1);
+            }
     }
 }
 
@@ -134,6 +143,7 @@ __device__ __forceinline__ void add_product(double &sum, float v, float, double 
     asm("{\n\t.reg .pred p;\n\tsetp.neu.f32 p, %1, 0f00000000;\n\t@p fma.rn.f64 %0, %2, %3, %0;\n\t}"
         : "+d"(sum) : "f"(v), "d"(static_cast<double>(v)), "d"(x));
 }
+// (for a scale that is neither 0 nor infinite nor NaN: v * s is zero when v is)
 __device__ __forceinline__ void add_product(double &sum, __nv_bfloat16 v, float s, double x) {
     asm("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %1, 0;\n\t@p fma.rn.f64 %0, %2, %3, %0;\n\t}"
         : "+d"(sum) : "r"(__bfloat16_as_ushort(v) & 0x7fffu), "d"(widen<double>(v, s)), "d"(x));

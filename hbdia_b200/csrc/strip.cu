@@ -87,20 +87,19 @@ size_t strip_bytes(int32_t numTiles) { return (static_cast<size_t>(numTiles) + 3
 void make_strips(DevicePlan &P, void *where) {
     P.strips = nullptr;
     P.stripGrid = 0;
-    P.uniformStrips = 0;
     int device = 0, sms = 0;
     check_cuda(cudaGetDevice(&device), "cudaGetDevice");
     check_cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device), "cudaDeviceGetAttribute");
     if (!enough_strips(P, sms)) return;
     const int32_t strips = (P.numTiles + 3) / 4;
     int4 *desc = static_cast<int4 *>(where);
-    int32_t *uniform = reinterpret_cast<int32_t *>(desc + strips);
-    check_cuda(cudaMemset(uniform, 0, sizeof(int32_t)), "cudaMemset(strips)");
+    int32_t *counts = reinterpret_cast<int32_t *>(desc + strips), found[2] = {0, 0};
+    check_cuda(cudaMemset(counts, 0, sizeof(found)), "cudaMemset(strips)");
     dev::strip_desc_kernel<<<static_cast<unsigned>((strips + 7) / 8), 256>>>(
-        P.blkOff, P.offs, P.cooTile, P.numBlocks, P.numTiles, P.bw / 32, P.nCoo > 0, desc, uniform);
+        P.blkOff, P.offs, P.cooTile, P.scale, P.numBlocks, P.numTiles, P.bw / 32, P.nCoo > 0, desc, counts);
     check_cuda(cudaGetLastError(), "strip descriptors");
-    check_cuda(cudaMemcpy(&P.uniformStrips, uniform, sizeof(int32_t), cudaMemcpyDeviceToHost), "cudaMemcpy(strips)");
-    if (P.uniformStrips < kUniformShare * strips) return;
+    check_cuda(cudaMemcpy(found, counts, sizeof(found), cudaMemcpyDeviceToHost), "cudaMemcpy(strips)");
+    if (found[0] < kUniformShare * strips || found[1] != 0) return;
     P.strips = desc;
     P.stripGrid = static_cast<int32_t>(std::min<int64_t>((strips + kStripWarps - 1) / kStripWarps, sms));
     // here and not at the launch, which may be captured into a graph
