@@ -55,7 +55,8 @@ UNIT = "GB/s"
 KERNEL_NAMES = {1: "spmv_rowwise<double,double>", 2: "spmv_bw32<double,double>",
                 3: "spmv_bw32_xs<double,double> (x window staged by bulk copies)",
                 4: "spmv_bw32_pipe<double,double> (persistent, pipelined)",
-                5: "spmv_bw32_quad<double,double> (4 blocks per warp)"}
+                5: "spmv_bw32_quad<double,double> (4 blocks per warp)",
+                6: "spmv_strip<double,double> (128 rows per warp, values streamed through shared memory)"}
 
 
 def log(*a):
@@ -339,7 +340,7 @@ def main():
     ap.add_argument("--serve-requests", type=int, default=10000, help="Poisson requests per server (config 5)")
     ap.add_argument("--unroll", type=int, default=0, choices=[0, 9, 27],
                     help="offsets in flight per lane in the staged kernel (0: default)")
-    ap.add_argument("--kernel", default=None, choices=["pipe", "quad", "staged", "warp", "rowwise"],
+    ap.add_argument("--kernel", default=None, choices=["strip", "pipe", "quad", "staged", "warp", "rowwise"],
                     help="force one SpMV kernel (default: the library's choice)")
     ap.add_argument("--size", type=int, default=256,
                     help="grid edge of the stencil workload (256 is the benchmark; smaller sizes for profiling)")
@@ -370,7 +371,7 @@ def main():
     bytes_per_spmv = hbm_bytes_model(info)
     assert bytes_per_spmv == info.bytesPerSpmv, (bytes_per_spmv, info.bytesPerSpmv)
     if args.kernel:
-        m.setKernel({"pipe": hb.KERNEL_PIPE, "quad": hb.KERNEL_QUAD, "staged": hb.KERNEL_STAGED, "warp": hb.KERNEL_WARP,
+        m.setKernel({"pipe": hb.KERNEL_PIPE, "quad": hb.KERNEL_QUAD, "strip": hb.KERNEL_STRIP, "staged": hb.KERNEL_STAGED, "warp": hb.KERNEL_WARP,
                      "rowwise": hb.KERNEL_ROWWISE}[args.kernel])
     if args.unroll:
         m.setTuning(hb.TUNE_UNROLL, args.unroll)

@@ -18,7 +18,7 @@ from typing import List, Optional, Sequence
 import numpy as np
 
 from . import _lib
-from ._lib import (BATCH_CONCURRENT, BATCH_QUEUE, REQ_CG, REQ_SPMV, KERNEL_AUTO, KERNEL_PIPE, KERNEL_QUAD, KERNEL_ROWWISE, KERNEL_STAGED, KERNEL_WARP, TUNE_PREFETCH, TUNE_QUAD_GROUP, TUNE_SPMM_TILE, TUNE_STAGES, TUNE_TAIL,
+from ._lib import (BATCH_CONCURRENT, BATCH_QUEUE, REQ_CG, REQ_SPMV, KERNEL_AUTO, KERNEL_PIPE, KERNEL_QUAD, KERNEL_ROWWISE, KERNEL_STAGED, KERNEL_STRIP, KERNEL_WARP, TUNE_PREFETCH, TUNE_QUAD_GROUP, TUNE_SPMM_TILE, TUNE_STAGES, TUNE_TAIL,
                    TUNE_UNROLL, HBDIACudaError,
                    HBDIADeviceTimeout, STORE_BF16_SCALED, STORE_F32, STORE_NATIVE, STORE_F32_QUAD, STORE_BF16_QUAD, MatrixInfo,
                    check as _check, load as _load)
@@ -270,7 +270,7 @@ class HBDIA:
         return b.value
 
     def setKernel(self, kernel: int) -> None:
-        """KERNEL_AUTO / KERNEL_ROWWISE / KERNEL_WARP / KERNEL_STAGED."""
+        """KERNEL_AUTO / ROWWISE / WARP / STAGED / PIPE / QUAD / STRIP."""
         _check(_load().hbdia_matrix_set_kernel(self._h, int(kernel)))
 
     def selectedKernel(self, x_ptr: int) -> int:
@@ -540,6 +540,11 @@ class LayoutPlan:
 
     def spmv(self, x_ptr: int, y_ptr: int, stream: Optional[int] = None) -> None:
         _check(_load().hbdia_plan_spmv(self._h, ctypes.c_void_p(x_ptr), ctypes.c_void_p(y_ptr), _stream_arg(stream)))
+
+    def selectedKernel(self, x_ptr: int) -> int:
+        k = ctypes.c_int32(0)
+        _check(_load().hbdia_plan_selected_kernel(self._h, ctypes.c_void_p(x_ptr), ctypes.byref(k)))
+        return k.value
 
     def spmm(self, X_ptr: int, ldx: int, Y_ptr: int, ldy: int, k: int, stream: Optional[int] = None) -> None:
         _check(_load().hbdia_plan_spmm(self._h, ctypes.c_void_p(X_ptr), ldx, ctypes.c_void_p(Y_ptr), ldy, k,

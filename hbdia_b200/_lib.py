@@ -26,7 +26,7 @@ HBDIA_ERR_NOT_CONVERTED = -6
 HBDIA_ERR_UNSUPPORTED = -7
 HBDIA_ERR_DEVICE_TIMEOUT = -8
 
-KERNEL_AUTO, KERNEL_ROWWISE, KERNEL_WARP, KERNEL_STAGED, KERNEL_PIPE, KERNEL_QUAD = 0, 1, 2, 3, 4, 5
+KERNEL_AUTO, KERNEL_ROWWISE, KERNEL_WARP, KERNEL_STAGED, KERNEL_PIPE, KERNEL_QUAD, KERNEL_STRIP = 0, 1, 2, 3, 4, 5, 6
 TUNE_UNROLL, TUNE_SPMM_TILE, TUNE_PREFETCH, TUNE_TAIL, TUNE_STAGES, TUNE_QUAD_GROUP = 1, 2, 3, 4, 5, 6
 
 HBDIA_F64, HBDIA_F32 = 0, 1
@@ -218,6 +218,7 @@ _SIGS = [
     ("hbdia_plan_create", ctypes.c_int, [ctypes.POINTER(LayoutDesc), c_vpp]),
     ("hbdia_plan_spmv", ctypes.c_int, [c_vp, c_vp, c_vp, c_vp]),
     ("hbdia_plan_spmm", ctypes.c_int, [c_vp, c_vp, c_i64, c_vp, c_i64, c_i32, c_vp]),
+    ("hbdia_plan_selected_kernel", ctypes.c_int, [c_vp, c_vp, c_i32p]),
     ("hbdia_plan_destroy", None, [c_vp]),
     ("hbdia_server_submit_device", ctypes.c_int, [c_vp, c_i32, c_i32, c_vp, c_vp, ctypes.POINTER(ctypes.c_uint64)]),
 ]

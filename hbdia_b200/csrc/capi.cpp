@@ -582,7 +582,7 @@ int hbdia_matrix_device_status(const hbdia_matrix *m, int32_t *bits) {
 int hbdia_matrix_set_kernel(hbdia_matrix *m, int32_t kernel) {
     return guarded([&] {
         need(m != nullptr, HBDIA_ERR_INVALID_ARGUMENT, "null matrix");
-        need(kernel >= HBDIA_KERNEL_AUTO && kernel <= HBDIA_KERNEL_QUAD, HBDIA_ERR_INVALID_ARGUMENT,
+        need(kernel >= HBDIA_KERNEL_AUTO && kernel <= HBDIA_KERNEL_STRIP, HBDIA_ERR_INVALID_ARGUMENT,
              "unknown kernel");
         m->plan.kernel = kernel;
     });
@@ -1257,6 +1257,13 @@ int hbdia_plan_spmm(const hbdia_plan *p, const void *X, int64_t ldx, void *Y, in
     return guarded([&] {
         need(p != nullptr, HBDIA_ERR_INVALID_ARGUMENT, "null plan");
         hbdia::launch_spmm(p->P, X, ldx, Y, ldy, k, stream, false);
+    });
+}
+
+int hbdia_plan_selected_kernel(const hbdia_plan *p, const void *x, int32_t *kernel) {
+    return guarded([&] {
+        need(p && kernel, HBDIA_ERR_INVALID_ARGUMENT, "null argument");
+        *kernel = hbdia::select_kernel(p->P, x);
     });
 }
 

@@ -384,9 +384,6 @@ void launch_pipe(Kernel kernel, const dev::SpmvArgs<VT, XT> &a, int32_t numTiles
 // quad's values when x exceeds L2 (the pipelined kernel's rule).
 template <typename VT, typename XT>
 void launch_quad(const DevicePlan &P, const dev::SpmvArgs<VT, XT> &a, const XT *x, XT *y, cudaStream_t s) {
-    // narrow values without a knob set, wide blocks: the strip kernel where it pays
-    if (P.strips && (P.bw != 32 || (sizeof(VT) < sizeof(double) && P.dtype == HBDIA_F64 && !P.quadGroup && P.prefetchL2 < 0)))
-        return launch_strip<VT, XT>(P, x, y, s);
     int l2 = 0;
     const int device = plan_device(P);
     check_cuda(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, device), "cudaDeviceGetAttribute(L2)");
@@ -414,9 +411,6 @@ void launch_quad(const DevicePlan &P, const dev::SpmvArgs<VT, XT> &a, const XT *
 
 template <typename VT, typename XT>
 void launch_pipe_tuned(const DevicePlan &P, const dev::SpmvArgs<VT, XT> &a, const XT *x, XT *y, cudaStream_t s) {
-    // native values without a knob set: the strip kernel where it pays
-    if (P.strips && P.storage == HBDIA_STORE_NATIVE && P.prefetchL2 < 0 && P.maskedTail < 0 && P.unroll != 27)
-        return launch_strip<VT, XT>(P, x, y, s);
     // Forcing 4-6 CTAs per SM through __launch_bounds__ made ptxas spill and
     // ran 3-45% slower on B200; the compiler's own register choice is kept.
     // The prefetch pays when x does not fit in L2 (measured on B200: +1.5 % FP64
@@ -459,7 +453,8 @@ void launch_typed(const DevicePlan &P, const void *x, void *y, cudaStream_t s) {
         launch_pipe_tuned<VT, XT>(P, a, xp, yp, s);
     } else if (kern == HBDIA_KERNEL_QUAD) {
         launch_quad<VT, XT>(P, a, xp, yp, s);
-
+    } else if (kern == HBDIA_KERNEL_STRIP) {
+        launch_strip<VT, XT>(P, xp, yp, s);
     } else if (kern == HBDIA_KERNEL_WARP) {
         const int64_t warpsPerCta = 8;
         const unsigned grid = static_cast<unsigned>((P.numTiles + warpsPerCta - 1) / warpsPerCta);
@@ -481,7 +476,15 @@ int32_t iteration_storage(const HostLayout<double> &L, int32_t storage) {
 }
 
 int32_t select_kernel(const DevicePlan &P, const void *x) {
-    if (P.quadLayout) return HBDIA_KERNEL_QUAD;  // the only kernel that reads that layout
+    // AUTO runs the strip kernel on layouts where it is the faster one (strip.cu),
+    // unless a knob of the kernel it stands in for is set
+    const bool strip = P.strips && (P.kernel == HBDIA_KERNEL_STRIP ||
+                                    (P.kernel == HBDIA_KERNEL_AUTO &&
+                                     (P.bw != 32 || (P.prefetchL2 < 0 && (P.storage == HBDIA_STORE_NATIVE
+                                                                              ? P.maskedTail < 0 && P.unroll != 27
+                                                                              : !P.quadGroup)))));
+    if (strip) return HBDIA_KERNEL_STRIP;
+    if (P.quadLayout) return HBDIA_KERNEL_QUAD;  // the other kernel that reads that layout
     const bool bw32 = P.bw == 32;
     // the staged kernel bulk-copies x and the value slabs (16-byte aligned
     // starts), needs a status word for its bounded waits, and does row/column
@@ -499,16 +502,14 @@ int32_t select_kernel(const DevicePlan &P, const void *x) {
             if (pipeOk) return HBDIA_KERNEL_PIPE;
             return bw32 ? HBDIA_KERNEL_WARP : HBDIA_KERNEL_ROWWISE;
         case HBDIA_KERNEL_QUAD:
-            if (pipeOk || P.strips) return HBDIA_KERNEL_QUAD;
+            if (pipeOk) return HBDIA_KERNEL_QUAD;
             return bw32 ? HBDIA_KERNEL_WARP : HBDIA_KERNEL_ROWWISE;
         case HBDIA_KERNEL_WARP: return bw32 ? HBDIA_KERNEL_WARP : HBDIA_KERNEL_ROWWISE;
-        default:  // AUTO: the fastest measured on B200 for blockWidth 32
+        default:  // AUTO (or STRIP on a layout without strips): the fastest measured on B200 for blockWidth 32
             // (4- and 2-byte values: the quad kernel, 2-10 % ahead of the
             // pipelined one on the 27-point 128^3 and 256^3 workloads; FP64
             // values: the pipelined kernel, which the quad one trails there)
-            // (both run as the strip kernel on layouts where that pays: strip.cu)
             if (pipeOk) return P.storage == HBDIA_STORE_NATIVE ? HBDIA_KERNEL_PIPE : HBDIA_KERNEL_QUAD;
-            if (P.strips) return HBDIA_KERNEL_QUAD;  // wide blocks
             return bw32 ? HBDIA_KERNEL_WARP : HBDIA_KERNEL_ROWWISE;
     }
 }

@@ -656,7 +656,7 @@ def spmv(args):
     m = hb.HBDIA(rows, cols, vals, n, n)
     m.convertToHBDIAFormat(32, 2, upload=False)
     m.prepareForGPU(args.storage)
-    kern = {"auto": hb.KERNEL_AUTO, "pipe": hb.KERNEL_PIPE, "quad": hb.KERNEL_QUAD, "staged": hb.KERNEL_STAGED,
+    kern = {"auto": hb.KERNEL_AUTO, "pipe": hb.KERNEL_PIPE, "quad": hb.KERNEL_QUAD, "strip": hb.KERNEL_STRIP, "staged": hb.KERNEL_STAGED,
             "warp": hb.KERNEL_WARP, "rowwise": hb.KERNEL_ROWWISE}[args.kernel]
     m.setKernel(kern)
     x = torch.from_numpy(hb.fill_uniform(n, -1.0, 1.0, 1)).cuda()
@@ -701,7 +701,7 @@ def main(argv=None):
     ap.add_argument("--n", type=int, default=8 * 1024 * 1024)
     ap.add_argument("--grid", type=int, default=128)
     ap.add_argument("--device", action="store_true", help="serve: request vectors in device memory")
-    ap.add_argument("--kernel", default="auto", choices=["auto", "pipe", "quad", "staged", "warp", "rowwise"])
+    ap.add_argument("--kernel", default="auto", choices=["auto", "strip", "pipe", "quad", "staged", "warp", "rowwise"])
     ap.add_argument("--reps", type=int, default=20)
     ap.add_argument("--rhs", type=int, default=1, help="spmv: right-hand sides (> 1: column-major SpMM)")
     ap.add_argument("--tile", type=int, default=0, help="spmv --rhs: right-hand sides per pass (0: default)")

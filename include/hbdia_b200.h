@@ -57,7 +57,7 @@ typedef enum hbdia_exec_mode { HBDIA_CPU_COO = 0, HBDIA_GPU_COO = 1 } hbdia_exec
  * consecutive blocks with one list of at most 32 offsets) interleaved
  * [offset][lane][block], so that the quad kernel reads a lane's four values of
  * an offset with one 16- / 8-byte load; they need blockWidth 32, run the SpMV
- * through the quad kernel only (whatever kernel is set) and give the same y
+ * through the quad and strip kernels only (whatever kernel is set) and give the same y
  * as F32 / BF16_SCALED bit for bit; SpMM, vector lists and batches refuse
  * them (HBDIA_ERR_UNSUPPORTED). */
 typedef enum hbdia_value_storage {
@@ -69,14 +69,13 @@ typedef enum hbdia_value_storage {
 } hbdia_value_storage;
 
 /* SpMV kernel choice (all give bit-identical y).  AUTO picks the kernel
- * measured fastest on B200: for blockWidth 32 QUAD with 4- and 2-byte value
- * storage, PIPE with native values; for other block widths QUAD when it is a
- * multiple of 32 and the matrix is large and regular enough, else ROWWISE.
- * PIPE (native values), QUAD (narrow ones, and wide blocks) run as the strip
- * kernel, which streams the values of 4 blocks of 32 rows through shared
- * memory, on layouts where that is the faster form.  STAGED
- * needs a 16-byte aligned x and value array (else WARP runs); PIPE and STAGED
- * need numRows <= 2^30. */
+ * measured fastest on B200: STRIP for block widths that are multiples of 32
+ * when the matrix is large and regular enough and no tuning knob of PIPE
+ * (native values) or QUAD (narrow ones) is set; else for blockWidth 32 QUAD
+ * with 4- and 2-byte value storage and PIPE with native values, and ROWWISE for
+ * other block widths.  STRIP set on a layout where it does not pay runs what
+ * AUTO would.  STAGED needs a 16-byte aligned x and value array (else WARP
+ * runs); PIPE and STAGED need numRows <= 2^30. */
 typedef enum hbdia_kernel {
     HBDIA_KERNEL_AUTO = 0,
     HBDIA_KERNEL_ROWWISE = 1, /* one thread per row, any blockWidth             */
@@ -84,7 +83,8 @@ typedef enum hbdia_kernel {
     HBDIA_KERNEL_STAGED = 3,  /* persistent; each warp bulk-copies its next tiles' values and
                                  x runs into shared memory, blockWidth 32 */
     HBDIA_KERNEL_PIPE = 4,    /* persistent warp per block, pipelined across blocks, blockWidth 32 */
-    HBDIA_KERNEL_QUAD = 5     /* persistent warp per 4 blocks sharing one offset list, blockWidth 32 */
+    HBDIA_KERNEL_QUAD = 5,    /* persistent warp per 4 blocks sharing one offset list, blockWidth 32 */
+    HBDIA_KERNEL_STRIP = 6    /* persistent; each warp streams the values of 128 rows through shared memory */
 } hbdia_kernel;
 
 typedef struct hbdia_matrix hbdia_matrix; /* HBDIA<T>       (include/Format/HBDIA.hpp:24-291)      */
@@ -351,7 +351,8 @@ int hbdia_spmv_host_many(hbdia_matrix *m, const void *const *xHost, void *const 
  * The arrays prepareForGPU leaves on the device (src/Format/HBDIA.cpp:720-816),
  * read through the reference's getters (include/Format/HBDIA.hpp:155-165):
  *   values      getHBDIADataDevice()          totalOffsets * blockWidth, [block][offsetIdx][lane]
- *   offsets     getFlattenedOffsetsDevice()   totalOffsets, ascending within each block
+ *   offsets     getFlattenedOffsetsDevice()   totalOffsets, ascending within each block (in
+ *                                             another order they are summed in that order)
  *   blockStart  getBlockStartIndicesDevice()  numBlocks + 1, offset units
  *   cooRow, cooCol, cooVal, cooRowPtr         getCpuRowIndicesDevice() ... getCpuRowPtrDevice():
  *                                             numCoo entries, row-sorted; numRows + 1 row pointer
@@ -389,6 +390,8 @@ int hbdia_plan_spmv(const hbdia_plan *p, const void *x, void *y, void *stream);
 /* Y = A X, row-major blocks (as hbdia_spmm_device). */
 int hbdia_plan_spmm(const hbdia_plan *p, const void *X, int64_t ldx, void *Y, int64_t ldy, int32_t k,
                     void *stream);
+/* The kernel hbdia_plan_spmv would launch for this x pointer. */
+int hbdia_plan_selected_kernel(const hbdia_plan *p, const void *x, int32_t *kernel);
 void hbdia_plan_destroy(hbdia_plan *p);
 
 /* hbdia_spmv_host without any device allocation.  No counterpart in the
