@@ -199,7 +199,7 @@ void launch_spmm_tile(const DevicePlan &P, const void *X, int64_t ldx, void *Y, 
                       int32_t tile, void *stream, bool colMajor = false);
 int32_t default_spmm_tile(int32_t k, bool colMajor = false);
 // Row-major Y = A X in passes of up to `width` columns, blockWidth a multiple
-// of 32 and numRows <= 2^30 (spmm_rows.cu).
+// of 32, numRows <= 2^30, offsets ascending in every block (spmm_rows.cu).
 template <typename VT, typename XT>
 void launch_spmm_rows(const DevicePlan &P, const XT *X, int64_t ldx, XT *Y, int64_t ldy, int32_t k, int32_t width,
                       void *stream);

@@ -534,7 +534,7 @@ namespace {
 template <typename VT, typename XT, int KT, bool CM>
 void launch_spmm_kt(const DevicePlan &P, const dev::SpmvArgs<VT, XT> &a, const XT *X, int64_t ldx, XT *Y,
                     int64_t ldy, int32_t k, cudaStream_t s) {
-    if (P.bw == 32 && !CM) {  // only more than 2^30 rows come here: 64-bit indices
+    if (P.bw == 32 && !CM) {  // only more than 2^30 rows and lists that do not ascend come here
         const unsigned grid = static_cast<unsigned>((static_cast<int64_t>(P.numTiles) + 7) / 8);
         dev::spmm_bw32<VT, XT, KT, CM, int64_t, false><<<grid, 256, 0, s>>>(a, X, ldx, Y, ldy, k);
     } else if (P.bw == 32) {
@@ -579,7 +579,7 @@ void launch_spmm_typed(const DevicePlan &P, const void *X, int64_t ldx, void *Y,
     const XT *xp = static_cast<const XT *>(X);
     XT *yp = static_cast<XT *>(Y);
     if (colMajor) launch_spmm_layout<VT, XT, true>(P, a, xp, ldx, yp, ldy, k, tile, s);
-    else if (P.bw % 32 == 0 && P.n <= (1 << 30)) launch_spmm_rows<VT, XT>(P, xp, ldx, yp, ldy, k, tile, s);
+    else if (P.bw % 32 == 0 && P.n <= (1 << 30) && P.ascending) launch_spmm_rows<VT, XT>(P, xp, ldx, yp, ldy, k, tile, s);
     else launch_spmm_layout<VT, XT, false>(P, a, xp, ldx, yp, ldy, k, tile, s);
     check_cuda(cudaGetLastError(), "SpMM launch");
 }

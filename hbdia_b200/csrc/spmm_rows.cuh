@@ -20,6 +20,7 @@
 // shared memory (k = 16 197-207, k = 32 375, but float k = 16 149 against 115),
 // 4 rows a lane for 9 to 16 columns (258).
 //
+// Offsets ascend in every block (interior tiles are told by a list's ends).
 // Column j is computed with exactly the SpMV's arithmetic (spmv_kernels.cuh).
 #pragma once
 
@@ -172,7 +173,7 @@ __device__ __forceinline__ void rows_dia(const SpmvArgs<VT, XT> &a, const XT *__
         const int32_t o1 = __shfl_down_sync(kFull, myoff, 1), o2 = __shfl_down_sync(kFull, myoff, 2);
         const unsigned runs = __ballot_sync(kFull, lane + 2 < cnt && o1 == myoff + 1 && o2 == myoff + 2);
         const int32_t oF = __shfl_sync(kFull, myoff, 0), oL = __shfl_sync(kFull, myoff, cnt - 1);
-        const bool interior = a.ascending && int64_t(row0) + oF >= 0 && int64_t(row0) + RS - 1 + oL < int64_t(a.xn);
+        const bool interior = int64_t(row0) + oF >= 0 && int64_t(row0) + RS - 1 + oL < int64_t(a.xn);
         // L neighbouring offsets from j on (RUN: one after the other, so
         // that they share rows of X; else any)
         auto step = [&](auto LEN, auto RUNT, auto CHECK, int j) {

@@ -35,6 +35,8 @@
 // bulk L2 prefetch of the next strip's values (66 against 58), deeper rings
 // (6 stages 60 against 56: less L1 for x), 24 warps with 80 registers (spills).
 //
+// Offsets ascend in every block: a list's ends bound the others.
+//
 // Arithmetic is the reference's, in the reference's order: per row, offsets
 // ascending, stored zeros and columns outside [0, xn) skipped, fma; COO
 // products summed from zero in list order with separately rounded multiply
@@ -381,7 +383,7 @@ spmv_strip(const SpmvArgs<VT, XT> a, const int4 *__restrict__ desc, const XT *__
             }
         }
         if (K > 0) {
-            const bool interior = a.ascending && int64_t(row0) + so[0] >= 0 && int64_t(row0) + 127 + so[K - 1] < int64_t(a.xn);
+            const bool interior = int64_t(row0) + so[0] >= 0 && int64_t(row0) + 127 + so[K - 1] < int64_t(a.xn);
             // C offsets from g on: their x first, then their values
             auto step = [&](auto CNT, auto CHECK, int32_t g) {
                 constexpr int C = decltype(CNT)::value;

@@ -65,12 +65,14 @@ void configure(const DevicePlan &P) {
 //    96^3 (48 K) 17.3 -> 16.5;
 //  * wide blocks, from half a strip a warp: 27-point blockWidth 64 32^3 (0.1)
 //    12.4 -> 14.4, 45^3 (0.3) equal, 64^3 (0.9) 22.6 -> 20.7.
-// 16-byte copies need a 16-byte aligned value array (a caller's may not be).
+// 16-byte copies need a 16-byte aligned value array (a caller's may not be), and
+// the kernel ascending lists: a flag in it that turns the unchecked path off
+// instead cost 1.6 % of BF16 131x127x125 (59.9 -> 60.8 us).
 bool enough_strips(const DevicePlan &P, int sms) {
     const int64_t strips = (static_cast<int64_t>(P.numTiles) + 3) / 4, warps = int64_t(sms) * kStripWarps;
     const bool native = P.storage == HBDIA_STORE_NATIVE, bf16 = P.storage == HBDIA_STORE_BF16_SCALED;
     if (P.bw % 32 != 0 || P.n > (1 << 30) || (bf16 && P.bw != 32)) return false;
-    if ((reinterpret_cast<uintptr_t>(P.vals) & 15) != 0) return false;
+    if ((reinterpret_cast<uintptr_t>(P.vals) & 15) != 0 || !P.ascending) return false;
     if (native) return strips >= (P.bw != 32 ? warps / 2 : P.tailHeavy ? 2 * warps : 4 * warps);
     const int64_t stripOffsets = P.totalOffsets * (P.bw / 32) / 4;
     return bf16 ? strips >= warps * 3 / 2 && stripOffsets >= 48 * 1024 : strips >= warps / 2 && stripOffsets >= 32 * 1024;
