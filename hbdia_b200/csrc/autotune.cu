@@ -153,7 +153,7 @@ void autotune(DevicePlan &P, const void *X, int64_t ldx, void *Y, int64_t ldy, i
         if (!std::isfinite(bestMs)) {  // nothing eligible: keep the defaults
             best.kernel = keepKernel;
             best.unroll = keepUnroll;
-            best.tile = default_spmm_tile(k);
+            best.tile = default_spmm_tile(P, k);
         }
         std::lock_guard<std::mutex> lk(g_mu);
         g_table[key] = best;

@@ -197,7 +197,7 @@ void launch_spmm(const DevicePlan &P, const void *X, int64_t ldx, void *Y, int64
                  void *stream, bool colMajor = false);
 void launch_spmm_tile(const DevicePlan &P, const void *X, int64_t ldx, void *Y, int64_t ldy, int32_t k,
                       int32_t tile, void *stream, bool colMajor = false);
-int32_t default_spmm_tile(int32_t k, bool colMajor = false);
+int32_t default_spmm_tile(const DevicePlan &P, int32_t k, bool colMajor = false);
 // Row-major Y = A X in passes of up to `width` columns, blockWidth a multiple
 // of 32, numRows <= 2^30, offsets ascending in every block (spmm_rows.cu).
 template <typename VT, typename XT>

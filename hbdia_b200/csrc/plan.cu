@@ -572,6 +572,9 @@ void launch_spmm_layout(const DevicePlan &P, const dev::SpmvArgs<VT, XT> &a, con
     }
 }
 
+// Row-major blocks: lanes share rows of X (spmm_rows.cu).
+bool rows_shared(const DevicePlan &P) { return P.bw % 32 == 0 && P.n <= (1 << 30) && P.ascending; }
+
 template <typename VT, typename XT>
 void launch_spmm_typed(const DevicePlan &P, const void *X, int64_t ldx, void *Y, int64_t ldy, int32_t k,
                        int32_t tile, bool colMajor, cudaStream_t s) {
@@ -579,21 +582,27 @@ void launch_spmm_typed(const DevicePlan &P, const void *X, int64_t ldx, void *Y,
     const XT *xp = static_cast<const XT *>(X);
     XT *yp = static_cast<XT *>(Y);
     if (colMajor) launch_spmm_layout<VT, XT, true>(P, a, xp, ldx, yp, ldy, k, tile, s);
-    else if (P.bw % 32 == 0 && P.n <= (1 << 30) && P.ascending) launch_spmm_rows<VT, XT>(P, xp, ldx, yp, ldy, k, tile, s);
+    else if (rows_shared(P)) launch_spmm_rows<VT, XT>(P, xp, ldx, yp, ldy, k, tile, s);
     else launch_spmm_layout<VT, XT, false>(P, a, xp, ldx, yp, ldy, k, tile, s);
     check_cuda(cudaGetLastError(), "SpMM launch");
 }
 
 }  // namespace
 
-int32_t default_spmm_tile(int32_t k, bool colMajor) {
+int32_t default_spmm_tile(const DevicePlan &P, int32_t k, bool colMajor) {
     // Measured on B200 (27-point stencil 256^3): column-major blocks are
     // fastest in passes of 4 for every k >= 3 (each column a separate
-    // coalesced gather).  Row-major ones take whole rows of X, up to 32 columns
-    // a pass, so that every value is read once.
+    // coalesced gather).  Row-major ones take whole rows of X where lanes share
+    // them (spmm_rows.cuh), up to 32 columns a pass, so that every value is read
+    // once.  One row per thread (spmm_rowwise) is held back by its registers
+    // instead (FP64: 62 at 8 columns, 97 at 32): 27-point blockWidth 16 FP64 in
+    // passes of 8 against 16 or 32: 64^3 k = 16 434 against 474 us, k = 32 863
+    // against 982, 96^3 k = 32 2906 against 2948; float k = 32 978 against 887
+    // and 2909 against 2877, 16^3 k = 16 37.0 against 39.0.
     if (k <= 2) return 2;
     if (colMajor || k <= 4) return 4;
-    return k <= 8 ? 8 : k <= 16 ? 16 : 32;
+    if (rows_shared(P)) return k <= 8 ? 8 : k <= 16 ? 16 : 32;
+    return P.dtype == HBDIA_F32 && k > 16 ? 32 : 8;
 }
 
 void launch_spmm_tile(const DevicePlan &P, const void *X, int64_t ldx, void *Y, int64_t ldy, int32_t k,
@@ -662,7 +671,7 @@ void launch_spmv_list(const DevicePlan &P, const void *const *x, void *const *y,
     }
     for (int32_t j0 = 0; j0 < k; j0 += dev::kVecListMax) {
         const int32_t kk = std::min<int32_t>(dev::kVecListMax, k - j0);
-        const int32_t tile = P.spmmTileForced ? P.spmmTileForced : default_spmm_tile(kk, true);
+        const int32_t tile = P.spmmTileForced ? P.spmmTileForced : default_spmm_tile(P, kk, true);
         if (P.dtype == HBDIA_F32) launch_list_typed<float, float>(P, x + j0, y + j0, kk, tile, s);
         else if (P.storage == HBDIA_STORE_F32) launch_list_typed<float, double>(P, x + j0, y + j0, kk, tile, s);
         else if (P.storage == HBDIA_STORE_BF16_SCALED)
@@ -676,7 +685,7 @@ void launch_spmm(const DevicePlan &P, const void *X, int64_t ldx, void *Y, int64
     int32_t tile = P.spmmTileForced;
     if (!tile) {  // the autotuner's table is measured on row-major blocks
         auto it = colMajor ? P.spmmTile.end() : P.spmmTile.find(k);
-        tile = it != P.spmmTile.end() ? it->second : default_spmm_tile(k, colMajor);
+        tile = it != P.spmmTile.end() ? it->second : default_spmm_tile(P, k, colMajor);
     }
     launch_spmm_tile(P, X, ldx, Y, ldy, k, tile, stream, colMajor);
 }
