@@ -584,7 +584,20 @@ int hbdia_matrix_set_kernel(hbdia_matrix *m, int32_t kernel) {
         need(m != nullptr, HBDIA_ERR_INVALID_ARGUMENT, "null matrix");
         need(kernel >= HBDIA_KERNEL_AUTO && kernel <= HBDIA_KERNEL_STRIP, HBDIA_ERR_INVALID_ARGUMENT,
              "unknown kernel");
-        m->plan.kernel = kernel;
+        hbdia::DevicePlan &P = m->plan;
+        P.kernel = kernel;
+        if (kernel == HBDIA_KERNEL_STRIP && P.base && !P.strips) {  // a layout that AUTO runs without it
+            int device = 0;
+            hbdia::check_cuda(cudaGetDevice(&device), "cudaGetDevice");
+            if (P.device >= 0) hbdia::check_cuda(cudaSetDevice(P.device), "cudaSetDevice");
+            try {
+                hbdia::make_strips(P, P.stripMem);
+            } catch (...) {
+                cudaSetDevice(device);
+                throw;
+            }
+            cudaSetDevice(device);
+        }
     });
 }
 

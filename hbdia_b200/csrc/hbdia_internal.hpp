@@ -126,8 +126,9 @@ struct DevicePlan {
     void *cooVal = nullptr;              // T
     int32_t *cooRowPtr = nullptr, *cooTile = nullptr;
     bool ascending = true;               // every block's offsets ascend (a caller's may not: layout_plan.cu)
-    void *strips = nullptr;              // strip descriptors (spmv_strip.cuh); null: the strip kernel
-                                         // is not the faster one for this layout
+    void *stripMem = nullptr;            // where the strip descriptors (spmv_strip.cuh) go in the plan's allocation
+    void *strips = nullptr;              // they: made where the strip kernel pays, or when it is set
+    bool stripPays = false;              // it is the faster kernel for this layout: AUTO runs it
     int32_t stripGrid = 0;               // its CTAs
     void *stream = nullptr;              // cudaStream_t owned by the plan
     int32_t device = -1;                 // the device the layout lives on (current when it was built)
@@ -181,7 +182,7 @@ void borrow_plan(const hbdia_layout_desc &d, DevicePlan &P);
 void free_plan(DevicePlan &P);
 // Strip descriptors (strip.cu): their bytes in a plan's allocation, and making
 // them there from the layout on the device (P.strips: set where the strip
-// kernel pays).
+// kernel pays, or is set and can read the layout).
 size_t strip_bytes(int32_t numTiles);
 void make_strips(DevicePlan &P, void *where);
 template <typename VT, typename XT>

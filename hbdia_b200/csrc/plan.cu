@@ -479,7 +479,7 @@ int32_t select_kernel(const DevicePlan &P, const void *x) {
     // AUTO runs the strip kernel on layouts where it is the faster one (strip.cu),
     // unless a knob of the kernel it stands in for is set
     const bool strip = P.strips && (P.kernel == HBDIA_KERNEL_STRIP ||
-                                    (P.kernel == HBDIA_KERNEL_AUTO &&
+                                    (P.kernel == HBDIA_KERNEL_AUTO && P.stripPays &&
                                      (P.bw != 32 || (P.prefetchL2 < 0 && (P.storage == HBDIA_STORE_NATIVE
                                                                               ? P.maskedTail < 0 && P.unroll != 27
                                                                               : !P.quadGroup)))));

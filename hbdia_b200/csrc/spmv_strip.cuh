@@ -132,6 +132,28 @@ strip_desc_kernel(const int32_t *__restrict__ blkOff, const int32_t *__restrict_
     }
 }
 
+// *over += the warps of W whose share exceeds limit, in stored offsets of 32-row
+// tiles, a strip of differing tiles counted twice (its tiles go one by one).
+inline __global__ void __launch_bounds__(256)
+strip_share_kernel(const int4 *__restrict__ desc, const int32_t *__restrict__ blkOff, int32_t numBlocks, int32_t numTiles,
+                   int32_t tilesPerBlock, int32_t W, int32_t limit, int32_t *__restrict__ over) {
+    const int32_t w = static_cast<int32_t>(blockIdx.x) * 256 + threadIdx.x;
+    if (w >= W) return;
+    int32_t sum = 0;
+    for (int32_t s = w; s < (numTiles + 3) / 4; s += W) {
+        const int32_t K = desc[s].y;
+        if (K >= 0) {
+            sum += 4 * K;
+            continue;
+        }
+        for (int32_t t = s * 4; t < min(s * 4 + 4, numTiles); ++t) {
+            const int32_t b = t / tilesPerBlock;
+            if (b < numBlocks) sum += 2 * (blkOff[b + 1] - blkOff[b]);
+        }
+    }
+    if (sum > limit) atomicAdd(over, 1);
+}
+
 // sum += v * x unless the stored value is zero, as one predicated FMA.
 // For 8-byte values the product of a zero is made -0 instead, which leaves
 // every sum as it is: x keeps its low word and takes the zero's negative for

@@ -73,8 +73,9 @@ typedef enum hbdia_value_storage {
  * when the matrix is large and regular enough and no tuning knob of PIPE
  * (native values) or QUAD (narrow ones) is set; else for blockWidth 32 QUAD
  * with 4- and 2-byte value storage and PIPE with native values, and ROWWISE for
- * other block widths.  STRIP set on a layout where it does not pay runs what
- * AUTO would.  STAGED needs a 16-byte aligned x and value array (else WARP
+ * other block widths.  STRIP set on a layout that it cannot read (another block
+ * width, a value array off a 16-byte boundary, BF16 values in wide blocks or
+ * under a scale of 0 or infinity) runs what AUTO would.  STAGED needs a 16-byte aligned x and value array (else WARP
  * runs); PIPE and STAGED need numRows <= 2^30. */
 typedef enum hbdia_kernel {
     HBDIA_KERNEL_AUTO = 0,

@@ -69,14 +69,44 @@ def test_kernel_choice(lib, storage, dtype, bw):
 def test_small_layouts(lib):
     n = 4000
     rows, cols, vals = _banded(n, n, 3)
-    for bw, auto in ((32, lib.KERNEL_PIPE), (64, lib.KERNEL_ROWWISE)):
+    for bw, auto in ((32, lib.KERNEL_PIPE), (64, lib.KERNEL_ROWWISE), (48, lib.KERNEL_ROWWISE)):
         m = lib.HBDIA(rows, cols, vals, n, n)
         m.convertToHBDIAFormat(bw, 2)
         x = np.random.default_rng(1).uniform(-1, 1, n)
         y, k = _run(lib, m, x, lib.KERNEL_AUTO)
         assert k == auto
-        z, k = _run(lib, m, x, lib.KERNEL_STRIP)  # not there: as AUTO
+        z, k = _run(lib, m, x, lib.KERNEL_STRIP)  # runs where it can read the layout
+        assert k == (auto if bw == 48 else lib.KERNEL_STRIP) and bits_equal(z, y)
+        z, k = _run(lib, m, x, lib.KERNEL_AUTO)
         assert k == auto and bits_equal(z, y)
+
+
+@pytest.mark.parametrize("storage,dtype,bw,n,K", [
+    ("STORE_NATIVE", "f8", 32, 40000, 1), ("STORE_NATIVE", "f8", 32, 40077, 9), ("STORE_NATIVE", "f4", 32, 50001, 6), ("STORE_NATIVE", "f8", 64, 40045, 7),
+    ("STORE_NATIVE", "f8", 96, 60200, 4), ("STORE_NATIVE", "f4", 64, 50033, 31), ("STORE_F32", "f8", 32, 40045, 4), ("STORE_F32", "f8", 64, 40064, 8),
+    ("STORE_F32_QUAD", "f8", 32, 40045, 10), ("STORE_F32_QUAD", "f8", 32, 400031, 32), ("STORE_BF16_SCALED", "f8", 32, 40045, 7),
+    ("STORE_BF16_QUAD", "f8", 32, 40127, 13), ("STORE_BF16_SCALED", "f8", 32, 400000, 30)])
+def test_strip_set_equals_oracle(lib, orc, storage, dtype, bw, n, K):
+    """The strip kernel on every layout it can read: lists of every rest, strips
+    whose tiles differ, more than 32 offsets, stored zeros under an infinite or
+    NaN x, long COO rows."""
+    import oracle
+    from test_strip_gpu import _matrix
+    rows, cols, vals, x = _matrix(n, K, K + bw)
+    vals, x = vals.astype(dtype), x.astype(dtype)
+    m = lib.HBDIA(rows, cols, vals, n, n, dtype=np.dtype(dtype))
+    m.convertToHBDIAFormat(bw, 2, upload=False)
+    m.prepareForGPU(getattr(lib, storage))
+    ref = orc.convert(rows, cols, vals, n, n, bw, 2)
+    if storage == "STORE_NATIVE":
+        want = ref.spmv(x)
+    else:
+        L = ref.layout()
+        want = ref.spmv_with_values(L.data.astype(np.float32).astype(np.float64) if "F32" in storage else
+                                    oracle.bf16_block_scaled(L.data, L.block_start, bw), x)
+    y, k = _run(lib, m, x, lib.KERNEL_STRIP)
+    assert k == lib.KERNEL_STRIP
+    assert np.isfinite(want).all() and bits_equal(y, want)
 
 
 @pytest.mark.parametrize("shape", [(1.0, 0.8), (0.9, 1.0)])
@@ -140,3 +170,19 @@ def test_layout_plans(lib):
         torch.cuda.synchronize()
         ys.append(y)
     assert torch.equal(ys[0], ys[1])
+
+
+def test_uneven_shares(lib):
+    """Strips whose tiles differ that recur with a period of the warps' stride:
+    64^2 planes, 2 strips of 32, on the same warps every time."""
+    from hbdia_b200 import generate_stencil27
+    nz = -(-_rows(5) // 4096)
+    n = 64 * 64 * nz
+    rows, cols, vals = generate_stencil27(64, 64, nz, extra_fraction=0.002)
+    x = np.random.default_rng(1).uniform(-1, 1, n)
+    m = lib.HBDIA(rows, cols, vals, n, n)
+    m.convertToHBDIAFormat(32, 2)
+    y, k = _run(lib, m, x, lib.KERNEL_AUTO)
+    assert k == lib.KERNEL_PIPE
+    z, k = _run(lib, m, x, lib.KERNEL_STRIP)
+    assert k == lib.KERNEL_STRIP and bits_equal(z, y)
