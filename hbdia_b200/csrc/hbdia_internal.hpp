@@ -201,6 +201,8 @@ void launch_spmm_tile(const DevicePlan &P, const void *X, int64_t ldx, void *Y, 
 int32_t default_spmm_tile(const DevicePlan &P, int32_t k, bool colMajor = false);
 // Row-major Y = A X in passes of up to `width` columns, blockWidth a multiple
 // of 32, numRows <= 2^30, offsets ascending in every block (spmm_rows.cu).
+bool spmm_rows_wide(const void *X, int64_t ldx, const void *Y, int64_t ldy, int32_t k, int elem);
+bool spmm_rows_pay(const DevicePlan &P, int32_t k, bool wide, int64_t ldx);
 template <typename VT, typename XT>
 void launch_spmm_rows(const DevicePlan &P, const XT *X, int64_t ldx, XT *Y, int64_t ldy, int32_t k, int32_t width,
                       void *stream);

@@ -534,10 +534,7 @@ namespace {
 template <typename VT, typename XT, int KT, bool CM>
 void launch_spmm_kt(const DevicePlan &P, const dev::SpmvArgs<VT, XT> &a, const XT *X, int64_t ldx, XT *Y,
                     int64_t ldy, int32_t k, cudaStream_t s) {
-    if (P.bw == 32 && !CM) {  // only more than 2^30 rows and lists that do not ascend come here
-        const unsigned grid = static_cast<unsigned>((static_cast<int64_t>(P.numTiles) + 7) / 8);
-        dev::spmm_bw32<VT, XT, KT, CM, int64_t, false><<<grid, 256, 0, s>>>(a, X, ldx, Y, ldy, k);
-    } else if (P.bw == 32) {
+    if (P.bw == 32) {
         const unsigned grid = static_cast<unsigned>((static_cast<int64_t>(P.numTiles) + 7) / 8);
         // The full passes in one launch, a partial last pass (k not a multiple
         // of KT) in a second one on the remaining columns; 32-bit gather
@@ -547,12 +544,20 @@ void launch_spmm_kt(const DevicePlan &P, const dev::SpmvArgs<VT, XT> &a, const X
         const int32_t kfull = k - k % KT, krest = k % KT;
         const XT *Xr = CM ? X + static_cast<int64_t>(kfull) * ldx : X + kfull;
         XT *Yr = CM ? Y + static_cast<int64_t>(kfull) * ldy : Y + kfull;
-        if (i32) {
-            if (kfull) dev::spmm_bw32<VT, XT, KT, CM, int32_t, true><<<grid, 256, 0, s>>>(a, X, ldx, Y, ldy, kfull);
-            if (krest) dev::spmm_bw32<VT, XT, KT, CM, int32_t, false><<<grid, 256, 0, s>>>(a, Xr, ldx, Yr, ldy, krest);
-        } else {
+        // row-major blocks come here in passes of up to 8 columns, other widths and
+        // 64-bit indices are rare
+        if constexpr (CM || KT <= 8) {
+            if (i32) {
+                if (kfull) dev::spmm_bw32<VT, XT, KT, CM, int32_t, true><<<grid, 256, 0, s>>>(a, X, ldx, Y, ldy, kfull);
+                if (krest) dev::spmm_bw32<VT, XT, KT, CM, int32_t, false><<<grid, 256, 0, s>>>(a, Xr, ldx, Yr, ldy, krest);
+                return;
+            }
+        }
+        if constexpr (CM) {
             if (kfull) dev::spmm_bw32<VT, XT, KT, CM, int64_t, true><<<grid, 256, 0, s>>>(a, X, ldx, Y, ldy, kfull);
             if (krest) dev::spmm_bw32<VT, XT, KT, CM, int64_t, false><<<grid, 256, 0, s>>>(a, Xr, ldx, Yr, ldy, krest);
+        } else {
+            dev::spmm_bw32<VT, XT, KT, CM, int64_t, false><<<grid, 256, 0, s>>>(a, X, ldx, Y, ldy, k);
         }
     } else {
         const unsigned grid = static_cast<unsigned>((static_cast<int64_t>(P.n) + 255) / 256);
@@ -581,9 +586,10 @@ void launch_spmm_typed(const DevicePlan &P, const void *X, int64_t ldx, void *Y,
     dev::SpmvArgs<VT, XT> a = make_args<VT, XT>(P);
     const XT *xp = static_cast<const XT *>(X);
     XT *yp = static_cast<XT *>(Y);
-    if (colMajor) launch_spmm_layout<VT, XT, true>(P, a, xp, ldx, yp, ldy, k, tile, s);
-    else if (rows_shared(P)) launch_spmm_rows<VT, XT>(P, xp, ldx, yp, ldy, k, tile, s);
-    else launch_spmm_layout<VT, XT, false>(P, a, xp, ldx, yp, ldy, k, tile, s);
+    if (colMajor) launch_spmm_layout<VT, XT, true>(P, a, xp, ldx, yp, ldy, k, tile ? tile : default_spmm_tile(P, k, true), s);
+    else if (rows_shared(P) && spmm_rows_pay(P, k, spmm_rows_wide(X, ldx, Y, ldy, k, sizeof(XT)), ldx))
+        launch_spmm_rows<VT, XT>(P, xp, ldx, yp, ldy, k, tile ? tile : 32, s);
+    else launch_spmm_layout<VT, XT, false>(P, a, xp, ldx, yp, ldy, k, tile ? tile : default_spmm_tile(P, k), s);
     check_cuda(cudaGetLastError(), "SpMM launch");
 }
 
@@ -592,17 +598,16 @@ void launch_spmm_typed(const DevicePlan &P, const void *X, int64_t ldx, void *Y,
 int32_t default_spmm_tile(const DevicePlan &P, int32_t k, bool colMajor) {
     // Measured on B200 (27-point stencil 256^3): column-major blocks are
     // fastest in passes of 4 for every k >= 3 (each column a separate
-    // coalesced gather).  Row-major ones take whole rows of X where lanes share
-    // them (spmm_rows.cuh), up to 32 columns a pass, so that every value is read
-    // once.  One row per thread (spmm_rowwise) is held back by its registers
-    // instead (FP64: 62 at 8 columns, 97 at 32): 27-point blockWidth 16 FP64 in
-    // passes of 8 against 16 or 32: 64^3 k = 16 434 against 474 us, k = 32 863
-    // against 982, 96^3 k = 32 2906 against 2948; float k = 32 978 against 887
-    // and 2909 against 2877, 16^3 k = 16 37.0 against 39.0.
+    // coalesced gather), row-major ones with one lane per row in the smallest
+    // tile covering k up to 8 (wider passes re-fetch the same lines of X in every
+    // pass).  One row per thread (spmm_rowwise) is held back by its registers
+    // (FP64: 62 at 8 columns, 97 at 32): 27-point blockWidth 16 FP64 in passes of
+    // 8 against 16 or 32: 64^3 k = 16 434 against 474 us, k = 32 863 against 982,
+    // 96^3 k = 32 2906 against 2948; float k = 32 978 against 887 and 2909 against
+    // 2877, 16^3 k = 16 37.0 against 39.0.
     if (k <= 2) return 2;
     if (colMajor || k <= 4) return 4;
-    if (rows_shared(P)) return k <= 8 ? 8 : k <= 16 ? 16 : 32;
-    return P.dtype == HBDIA_F32 && k > 16 ? 32 : 8;
+    return P.bw != 32 && P.dtype == HBDIA_F32 && k > 16 ? 32 : 8;
 }
 
 void launch_spmm_tile(const DevicePlan &P, const void *X, int64_t ldx, void *Y, int64_t ldy, int32_t k,
@@ -682,10 +687,10 @@ void launch_spmv_list(const DevicePlan &P, const void *const *x, void *const *y,
 
 void launch_spmm(const DevicePlan &P, const void *X, int64_t ldx, void *Y, int64_t ldy, int32_t k, void *stream,
                  bool colMajor) {
-    int32_t tile = P.spmmTileForced;
-    if (!tile) {  // the autotuner's table is measured on row-major blocks
-        auto it = colMajor ? P.spmmTile.end() : P.spmmTile.find(k);
-        tile = it != P.spmmTile.end() ? it->second : default_spmm_tile(P, k, colMajor);
+    int32_t tile = P.spmmTileForced;  // 0: the kernel's default
+    if (!tile && !colMajor) {  // the autotuner's table is measured on row-major blocks
+        auto it = P.spmmTile.find(k);
+        if (it != P.spmmTile.end()) tile = it->second;
     }
     launch_spmm_tile(P, X, ldx, Y, ldy, k, tile, stream, colMajor);
 }

@@ -7,9 +7,11 @@
 // Here G lanes share a row of X and a lane keeps S neighbouring rows by V
 // columns: a request reads whole row segments, a lane's S values of one offset
 // are one or a few wide loads, and three neighbouring offsets (a stencil's -1,
-// 0, 1) read S + 2 rows of X instead of 3 S.  With one or two rows a lane, where
-// that saves little, 8 or 4 offsets' loads go out together instead.  Up to 32
-// columns a pass, so that the values are read once.
+// 0, 1) read S + 2 rows of X instead of 3 S.  Other offsets' loads go out
+// together too, 128 bytes of X a lane, the last ones of a list as groups of 4
+// and 1-3: one at a time each of them is a round trip (7-point 96^3 k = 2 67.9
+// -> 35.4 us, 27-point 96^3 k = 9 422 -> 252).  Up to 32 columns a pass, so that
+// the values are read once.
 //
 // B200, before -> after: 7-point 128^3 FP64 k = 16 603 -> 221 us, k = 32 1200 ->
 // 422, k = 5 341 -> 197; 27-point 128^3 k = 8 570 -> 338, k = 3 495 -> 253; 96^3
@@ -31,7 +33,7 @@
 namespace hbdia {
 namespace dev {
 
-constexpr int kRowsWarps = 16;  // warps per CTA
+constexpr int kRowsWarps = 16;  // warps per CTA at most (128 registers a thread)
 
 // N stored values from p on, p a multiple of their bytes up to 16 (vec) or of one value.
 template <typename VT, int N>
@@ -200,7 +202,7 @@ __device__ __forceinline__ void rows_dia(const SpmvArgs<VT, XT> &a, const XT *__
             // warp holds no stored zero among them.  With 8 rows a lane
             // the vote, which waits for all of them, costs more than the
             // tests (7-point 128^3 k = 16: 221 against 200 us).
-            constexpr int GL = S * L <= 12 ? L : 1;
+            constexpr int GL = S * L <= 16 ? L : 1;
             constexpr bool VOTE = !CK && S <= 4;
 #pragma unroll
             for (int l0 = 0; l0 < L; l0 += GL) {
@@ -241,24 +243,55 @@ __device__ __forceinline__ void rows_dia(const SpmvArgs<VT, XT> &a, const XT *__
             }
         };
         auto all = [&](auto CHECK) {
-            constexpr int U = S == 1 ? 8 : S == 2 ? 4 : 1;  // any offsets at once
+            // any offsets at once: 128 bytes of X a lane
+            constexpr int U = 128 / (S * V * static_cast<int>(sizeof(XT))) >= 8 ? 8 : 128 / (S * V * static_cast<int>(sizeof(XT)));
+            constexpr bool RUNS = S >= 4;
+            if constexpr (U == 1) {
+#pragma unroll 1
+                for (int j = 0; j < cnt;) {
+                    if (runs >> j & 1u) {
+                        step(std::integral_constant<int, 3>(), std::true_type(), CHECK, j);
+                        j += 3;
+                    } else {
+                        step(std::integral_constant<int, 1>(), std::false_type(), CHECK, j);
+                        ++j;
+                    }
+                }
+                return;
+            }
 #pragma unroll 1
             for (int j = 0; j < cnt;) {
-                if (U == 1 && (runs >> j & 1u)) {
+                const unsigned next = RUNS ? runs >> j : 0u;
+                if (next & 1u) {
                     step(std::integral_constant<int, 3>(), std::true_type(), CHECK, j);
                     j += 3;
-                } else if (U > 1 && j + U <= cnt) {
+                    continue;
+                }
+                // offsets before the next run: a group of U, else of 4, else the rest
+                const int left = next ? __ffs(next) - 1 : cnt - j;
+                if (left >= U) {
                     step(std::integral_constant<int, U>(), std::false_type(), CHECK, j);
                     j += U;
+                } else if (U > 4 && left >= 4) {
+                    step(std::integral_constant<int, U < 4 ? 1 : 4>(), std::false_type(), CHECK, j);
+                    j += 4;
                 } else {
-                    step(std::integral_constant<int, 1>(), std::false_type(), CHECK, j);
-                    ++j;
+                    if (U > 3 && left == 3) step(std::integral_constant<int, U < 3 ? 1 : 3>(), std::false_type(), CHECK, j);
+                    if (U > 2 && left == 2) step(std::integral_constant<int, U < 2 ? 1 : 2>(), std::false_type(), CHECK, j);
+                    if (U > 1 && left == 1) step(std::integral_constant<int, 1>(), std::false_type(), CHECK, j);
+                    j += left;
                 }
             }
         };
         if (interior) all(std::false_type());
         else all(std::true_type());
     }
+}
+
+// Instances whose CTAs always have kRowsWarps warps.
+template <typename XT, int V, int S>
+__host__ __device__ constexpr bool rows_fixed_cta() {
+    return S == 8 && V * sizeof(XT) == 16;
 }
 
 // One warp per slab of RS = (32 / G) S rows of a 32-row tile and C = G V
@@ -277,10 +310,13 @@ spmm_rows(const SpmvArgs<VT, XT> a, const XT *__restrict__ X, int64_t ldx, XT *_
     const int lane = threadIdx.x & 31;
     const int grp = lane / G;
     const int c = (lane % G) * V;
-    const int32_t W = static_cast<int32_t>(gridDim.x) * kRowsWarps;
+    // (a constant where registers are scarce: 8 rows of 16 bytes a lane spill 44
+    // bytes instead of 20 otherwise, 27-point 96^3 k = 16 258 -> 282 us)
+    const int32_t warps = rows_fixed_cta<XT, V, S>() ? kRowsWarps : static_cast<int32_t>(blockDim.x >> 5);
+    const int32_t W = static_cast<int32_t>(gridDim.x) * warps;
     const int32_t numSlabs = a.numTiles * HALVES;
     const int32_t m = a.bw >> 5;
-    int32_t s = static_cast<int32_t>(blockIdx.x) * kRowsWarps + (threadIdx.x >> 5);
+    int32_t s = static_cast<int32_t>(blockIdx.x) * warps + (threadIdx.x >> 5);
     if (s >= numSlabs) return;  // warp-uniform
 
     auto loadMeta = [&](int32_t q) {
