@@ -5,7 +5,7 @@
 // caller's own buffers and stream and keeps the fastest in the matrix's plan.
 // A process-wide table keyed on the matrix's shape class -- block width,
 // stored offsets per block, COO fraction, number of right-hand sides, value
-// type and storage -- lets later matrices of the same class take the choice
+// type and storage, and what of its size decides between kernels -- lets later matrices of the same class take the choice
 // without timing.
 
 #include <cuda_runtime.h>
@@ -22,7 +22,7 @@
 namespace hbdia {
 namespace {
 
-using Key = std::tuple<int32_t, int32_t, int32_t, int32_t, int32_t, int32_t>;
+using Key = std::tuple<int32_t, int32_t, int32_t, int32_t, int32_t, int32_t, int32_t>;
 
 struct Choice {
     int32_t kernel = HBDIA_KERNEL_AUTO;
@@ -46,7 +46,13 @@ Key key_of(const DevicePlan &P, int32_t k) {
     const double cooFrac = P.slots + P.nCoo > 0 ? double(P.nCoo) / double(P.slots + P.nCoo) : 0.0;
     // COO fraction bucket: 0, (0, 0.1%], (0.1%, 1%], (1%, 10%], > 10%
     const int32_t cooBucket = cooFrac == 0 ? 0 : cooFrac <= 1e-3 ? 1 : cooFrac <= 1e-2 ? 2 : cooFrac <= 0.1 ? 3 : 4;
-    return Key(P.bw, offsPerBlock, cooBucket, k_bucket(k), P.dtype, P.storage);
+    // the kernels in question depend on the layout's size and regularity: whether
+    // the strip kernel is among them (SpMV), the power of two of its rows (SpMM)
+    int32_t size = 0;
+    if (k == 1) size = P.stripPays ? 1 : 0;
+    else
+        while ((int64_t(1) << size) < P.n) ++size;
+    return Key(P.bw, offsPerBlock, cooBucket, k_bucket(k), P.dtype, P.storage, size);
 }
 
 void apply(DevicePlan &P, int32_t k, const Choice &c) {

@@ -468,7 +468,8 @@ int hbdia_matrix_set_tuning(hbdia_matrix *m, int32_t key, int32_t value);
  * (k > 1: RHS tile 4/8/16/32) on the given device buffers and stream, keeps
  * the fastest for the matrix, and records it in a process-wide table keyed on
  * (blockWidth, stored offsets per block, COO fraction, k, value type,
- * storage) so later matrices of the same class skip the timing (force != 0
+ * storage, whether the strip kernel pays (SpMV), the rows' power of two
+ * (SpMM)) so later matrices of the same class skip the timing (force != 0
  * times again).  All candidates give bit-identical results.  Overwrites Y. */
 typedef struct hbdia_tune_result {
     int32_t kernel;     /* hbdia_kernel chosen for k == 1   */

@@ -186,3 +186,23 @@ def test_uneven_shares(lib):
     assert k == lib.KERNEL_PIPE
     z, k = _run(lib, m, x, lib.KERNEL_STRIP)
     assert k == lib.KERNEL_STRIP and bits_equal(z, y)
+
+
+def test_autotuner_tells_sizes_apart(lib):
+    """A small matrix's choice is not taken by a large one of the same class that
+    the strip kernel can serve."""
+    import torch
+    lib.autotune_clear()
+    got = []
+    for n in (4000, _rows(8), _rows(9)):
+        rows, cols, vals = _banded(n, n, 3)
+        m = lib.HBDIA(rows, cols, vals, n, n)
+        m.convertToHBDIAFormat(64, 2)
+        x, y = torch.rand(n, dtype=torch.float64, device="cuda"), torch.zeros(n, dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        r = m.autotune(x.data_ptr(), y.data_ptr())
+        m.synchronize()
+        got.append((r.kernel, r.fromCache))
+        assert m.selectedKernel(x.data_ptr()) == r.kernel
+    assert got == [(lib.KERNEL_ROWWISE, 0), (lib.KERNEL_STRIP, 0), (lib.KERNEL_STRIP, 1)]
+    lib.autotune_clear()
