@@ -20,6 +20,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <vector>
 
 #include "hbdia_internal.hpp"
 
@@ -62,15 +63,24 @@ __global__ void check_layout(const int32_t *__restrict__ blk, int32_t nb, int64_
     if (f) atomicOr(flags, f);
 }
 
-// *flags |= 1 when some block's offsets do not ascend.
-__global__ void check_order(const int32_t *__restrict__ blk, const int32_t *__restrict__ offs, int32_t nb,
-                            int32_t *__restrict__ flags) {
+// lists[d]: blocks with d offsets (the last entry also those with more);
+// lists[kLists] != 0 when some block's offsets do not ascend.
+constexpr int kLists = 128;
+__global__ void __launch_bounds__(256) check_lists(const int32_t *__restrict__ blk, const int32_t *__restrict__ offs,
+                                                   int32_t nb, int32_t *__restrict__ lists) {
+    __shared__ int32_t h[kLists];
+    if (threadIdx.x < kLists) h[threadIdx.x] = 0;
+    __syncthreads();
     const int64_t b = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (b >= nb) return;
-    int32_t f = 0;
-    const int32_t k1 = blk[b + 1];
-    for (int32_t k = blk[b] + 1; k < k1; ++k) f |= offs[k - 1] > offs[k];
-    if (f) atomicOr(flags, 1);
+    if (b < nb) {
+        const int32_t k0 = blk[b], k1 = blk[b + 1];
+        atomicAdd(&h[min(k1 - k0, kLists - 1)], 1);
+        int32_t f = 0;
+        for (int32_t k = k0 + 1; k < k1; ++k) f |= offs[k - 1] > offs[k];
+        if (f) atomicOr(lists + kLists, 1);
+    }
+    __syncthreads();
+    if (threadIdx.x < kLists && h[threadIdx.x]) atomicAdd(lists + threadIdx.x, h[threadIdx.x]);
 }
 
 // cooTile[t] = rowPtr[min(32 t, n)]: the COO range of each 32-row tile.
@@ -131,7 +141,7 @@ void borrow_plan(const hbdia_layout_desc &d, DevicePlan &P) {
     const size_t oTile = 0;
     const size_t oStatus = up256((static_cast<size_t>(Q.numTiles) + 1) * sizeof(int32_t));
     const size_t oFlags = oStatus + 256;
-    const size_t oStrips = oFlags + 256;
+    const size_t oStrips = oFlags + up256((kLists + 1) * sizeof(int32_t));
     Q.bytes = oStrips + strip_bytes(Q.numTiles);
     check_cuda(dev_alloc(&Q.base, Q.bytes), "cudaMalloc(plan)");
     try {
@@ -156,11 +166,15 @@ void borrow_plan(const hbdia_layout_desc &d, DevicePlan &P) {
         tile_ranges<<<static_cast<unsigned>((Q.numTiles + 1 + 255) / 256), 256>>>(Q.cooRowPtr, Q.n, Q.numTiles,
                                                                                   Q.nCoo > 0, Q.cooTile);
         check_cuda(cudaGetLastError(), "tile_ranges");
-        if (Q.numBlocks > 0) {  // (the flags are all zero here, and the block starts valid)
-            check_order<<<static_cast<unsigned>((Q.numBlocks + 255) / 256), 256>>>(Q.blkOff, Q.offs, Q.numBlocks, flags);
-            check_cuda(cudaGetLastError(), "check_order");
-            check_cuda(cudaMemcpy(&f, flags, sizeof(int32_t), cudaMemcpyDeviceToHost), "cudaMemcpy(flags)");
-            Q.ascending = f == 0;
+        if (Q.numBlocks > 0) {  // (the block starts are valid here)
+            std::vector<int32_t> hist(kLists + 1);
+            check_cuda(cudaMemset(flags, 0, hist.size() * sizeof(int32_t)), "cudaMemset(lists)");
+            check_lists<<<static_cast<unsigned>((Q.numBlocks + 255) / 256), 256>>>(Q.blkOff, Q.offs, Q.numBlocks, flags);
+            check_cuda(cudaGetLastError(), "check_lists");
+            check_cuda(cudaMemcpy(hist.data(), flags, hist.size() * sizeof(int32_t), cudaMemcpyDeviceToHost), "cudaMemcpy(lists)");
+            Q.ascending = hist.back() == 0;
+            hist.pop_back();
+            Q.tailHeavy = tail_heavy(hist);
         }
         make_strips(Q, base + oStrips);
         cudaStream_t s;

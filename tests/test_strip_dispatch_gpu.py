@@ -206,3 +206,28 @@ def test_autotuner_tells_sizes_apart(lib):
         assert m.selectedKernel(x.data_ptr()) == r.kernel
     assert got == [(lib.KERNEL_ROWWISE, 0), (lib.KERNEL_STRIP, 0), (lib.KERNEL_STRIP, 1)]
     lib.autotune_clear()
+
+
+def test_layout_plan_of_short_lists(lib):
+    """Lists that are mostly tails of the pipelined kernel's groups reach the strip
+    kernel at the same size through a layout plan as through a matrix."""
+    import torch
+    n, offs = _rows(3), np.array([-700, -40, -1, 0, 1, 40, 700])
+    rows, cols, vals = _banded(n, n, 6, offs)
+    m = lib.HBDIA(rows, cols, vals, n, n)
+    m.convertToHBDIAFormat(32, 2)
+    L = m.layout()
+    dev = {k: torch.from_numpy(np.ascontiguousarray(L[k])).cuda() for k in ("data", "offsets", "block_start", "coo_row", "coo_col", "coo_val",
+                                                                            "coo_row_ptr")}
+    x = torch.rand(n, dtype=torch.float64, device="cuda")
+    y, z = torch.zeros_like(x), torch.zeros_like(x)
+    torch.cuda.synchronize()
+    p = lib.LayoutPlan(numRows=n, numCols=n, blockWidth=32, numBlocks=L["num_blocks"], totalOffsets=len(L["offsets"]), numCoo=len(L["coo_row"]),
+                       values=dev["data"].data_ptr(), offsets=dev["offsets"].data_ptr(), blockStart=dev["block_start"].data_ptr(),
+                       cooRow=dev["coo_row"].data_ptr(), cooCol=dev["coo_col"].data_ptr(), cooVal=dev["coo_val"].data_ptr(),
+                       cooRowPtr=dev["coo_row_ptr"].data_ptr(), keep=dev)
+    assert p.selectedKernel(x.data_ptr()) == m.selectedKernel(x.data_ptr()) == lib.KERNEL_STRIP
+    p.spmv(x.data_ptr(), y.data_ptr(), 0)
+    lib.spmv_device(m, x.data_ptr(), z.data_ptr(), 0)
+    torch.cuda.synchronize()
+    assert torch.equal(y, z)
