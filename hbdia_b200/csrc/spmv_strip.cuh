@@ -65,17 +65,6 @@ template <int N>
 __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
-// at most `pending` (0 .. N) of this thread's groups still in flight
-template <int N>
-__device__ __forceinline__ void cp_async_wait_upto(int pending) {
-    if constexpr (N == 0) {
-        cp_async_wait<0>();
-    } else {
-        if (pending >= N) cp_async_wait<N>();
-        else cp_async_wait_upto<N - 1>(pending);
-    }
-}
-
 // N list entries, four at a time; the list is 16-byte aligned there.
 template <int N>
 __device__ __forceinline__ void load_list(const int32_t *p, int32_t (&o)[N]) {
