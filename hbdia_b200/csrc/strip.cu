@@ -76,11 +76,15 @@ void configure(const DevicePlan &P) {
 //  * quad-interleaved FP32, a strip and 2.25: 27-point 64^3 (0.9) 13.3 -> 14.4,
 //    72^3 (1.2) 24.4 -> 20.7; short lists 2.25 and 1.75: 9 offsets 600 K
 //    (2.0) 10.3 -> 12.3, 800 K (2.6) 15.2 -> 15.0, 7-point 90^3 (2.4) 16.4 -> 14.4;
-//  * BF16 storage, either order, 2.75 and 1.6: 27-point 88^3 (2.2) 29.3 -> 30.8,
+//  * BF16 storage, 2.75 and 1.6: 27-point 88^3 (2.2) 29.3 -> 30.8,
 //    96^3 (2.9; 1.22) 32.7 -> 30.8, 104^3 (1.55) 48.4 -> 46.9, 300x10x650 (1.38)
 //    79.6 -> 82.6, 300x9x700 (1.46) 74.5 -> 66.8, 64x64x400 (1.87) 87.6 -> 96.6;
 //    short lists 4 and 1.5: 9 offsets 1 M rows (3.3) 18.4 -> 19.8, 1.5 M (4.9)
 //    23.1 -> 22.6, 7-point 104^3 (3.7; 1.59) 22.6 -> 24.6, 112^3 (4.6) 22.6 -> 22.4;
+//  * quad-interleaved BF16, 2.75 and 1.35: 27-point 88^3 32.5 -> 32.7, 96^3 33.0 ->
+//    32.6, 104^3 47.8 -> 49.2, 112^3 (1.20) 52.5 -> 45.3, 300x10x650 85.2 -> 88.6;
+//    short lists 4.5 and 1.5: 9 offsets 1.25 M rows (4.1) 22.6 -> 23.5, 1.5 M 24.0
+//    -> 23.4, 7-point 112^3 (4.6) 24.1 -> 23.4;
 //  * wide blocks (against one row per thread), half a strip (4-byte x 3/4) and 2.25:
 //    27-point blockWidth 64 FP64 45^3 (0.3) 14.4 -> 15.9, 54^3 (0.5) 18.9 -> 16.0,
 //    float 54^3 11.9 -> 12.3, 64^3 (0.9) 14.2 -> 12.5; short lists 1.5 and 1.65:
@@ -95,7 +99,10 @@ StripRule strip_rule(const DevicePlan &P) {
     const bool isLong = P.totalOffsets >= 16 * static_cast<int64_t>(P.numBlocks);
     if (P.bw != 32) return isLong ? StripRule{P.dtype == HBDIA_F32 ? 0.75 : 0.5, 2.25} : StripRule{1.5, 1.65};
     if (P.storage == HBDIA_STORE_NATIVE) return P.tailHeavy ? StripRule{2.0, 1.75} : StripRule{4.0, 1.33};
-    if (P.storage == HBDIA_STORE_BF16_SCALED) return isLong ? StripRule{2.75, 1.6} : StripRule{4.0, 1.5};
+    if (P.storage == HBDIA_STORE_BF16_SCALED) {
+        if (P.quadLayout) return isLong ? StripRule{2.75, 1.35} : StripRule{4.5, 1.5};
+        return isLong ? StripRule{2.75, 1.6} : StripRule{4.0, 1.5};
+    }
     if (P.quadLayout) return isLong ? StripRule{1.0, 2.25} : StripRule{2.25, 1.75};
     return isLong ? StripRule{0.55, 2.25} : StripRule{2.0, 2.0};
 }
