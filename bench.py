@@ -473,8 +473,7 @@ def main():
             "config": dict(workload_config(), parallelism=f"replicas{world}"),
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": profiled_traffic(), "peak_source": peak_kind,
-                         "traffic_source": "ncu dram__bytes_read+write of one 128^3 launch of the same kernel, "
-                                           "scaled to 256^3 by the byte model (profiles/)",
+                         "traffic_source": "ncu dram__bytes_read+write of one 256^3 launch of spmv_strip (profiles/)",
                          "kernel": KERNEL_NAMES[kernel_used], "bytes_per_launch": bytes_per_spmv,
                          "avg_launch_ms": avg_launch_ms},
             "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": 8 * n, "d2h_bytes_per_step": 8 * n,
