@@ -73,9 +73,13 @@ void configure(const DevicePlan &P) {
 //    64x64x400 (1.87) 99.0 -> 79.2; short ones 2 strips and 2: 9 offsets 560 K
 //    rows (1.85) 11.4 -> 12.3, 650 K (2.1) 14.9 -> 14.5, 7-point 85^3 (2.0) 15.9 ->
 //    14.4;
-//  * quad-interleaved FP32, a strip and 2.25: 27-point 64^3 (0.9) 13.3 -> 14.4,
-//    72^3 (1.2) 24.4 -> 20.7; short lists 2.25 and 1.75: 9 offsets 600 K
-//    (2.0) 10.3 -> 12.3, 800 K (2.6) 15.2 -> 15.0, 7-point 90^3 (2.4) 16.4 -> 14.4;
+//  * quad-interleaved FP32, which CG iterates on, half a strip and 32 K
+//    strip-offsets whatever the shares: between a CG's vector kernels the strip
+//    kernel is the faster one from there (solves of 27-point 56^3 6.5 -> 5.8 ms,
+//    64^3 6.9 -> 6.1, 70^3 9.0 -> 7.8, 72^3 and up equal or better), though lone
+//    products back to back are not before a strip a warp (56^3 12.3 -> 14.4 us,
+//    64^3 13.3 -> 14.4, 72^3 24.4 -> 20.7; 9 offsets 600 K rows 11.2 -> 12.3, 800 K
+//    15.2 -> 15.0);
 //  * BF16 storage, 2.75 and 1.6: 27-point 88^3 (2.2) 29.3 -> 30.8,
 //    96^3 (2.9; 1.22) 32.7 -> 30.8, 104^3 (1.55) 48.4 -> 46.9, 300x10x650 (1.38)
 //    79.6 -> 82.6, 300x9x700 (1.46) 74.5 -> 66.8, 64x64x400 (1.87) 87.6 -> 96.6;
@@ -103,7 +107,7 @@ StripRule strip_rule(const DevicePlan &P) {
         if (P.quadLayout) return isLong ? StripRule{2.75, 1.35} : StripRule{4.5, 1.5};
         return isLong ? StripRule{2.75, 1.6} : StripRule{4.0, 1.5};
     }
-    if (P.quadLayout) return isLong ? StripRule{1.0, 2.25} : StripRule{2.25, 1.75};
+    if (P.quadLayout) return StripRule{0.5, 1e9};
     return isLong ? StripRule{0.55, 2.25} : StripRule{2.0, 2.0};
 }
 
